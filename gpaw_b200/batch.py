@@ -3,9 +3,9 @@ one GPU.
 
 Each grid gets its own solver: its own device-resident level hierarchy,
 buffers and captured V-cycle loop (the whole solve runs on the device, see
-gb_poisson_* / gb_mixed_*).  A mixed-precision batch is, by default, ONE
-CUDA graph with a branch per grid (gb_mixed_batch_*): a single launch runs
-every solve, the branches side by side.  Otherwise (FP64, or graph=False)
+gb_poisson_* / gb_mixed_*).  A mixed batch is, by default, ONE CUDA graph
+(gb_mixed_batch_*): with the direct correction each kernel works on every
+grid at once, with V-cycles the graph has a branch per grid.  Otherwise (FP64, or graph=False)
 the batch enqueues every solve on one of ``nstreams`` CUDA streams.  Either
 way there is no host synchronisation until the results are read.
 """

@@ -9,6 +9,9 @@
 //       phi += e                     (FP64 accumulate, fused in the last sweep)
 //       d = rho - L64 phi
 //
+// Where the level-0 operator is separable, e is the direct FP64 correction of
+// gb_direct.cu instead of V32(d) (gb_mixed_set_direct).
+//
 // V32 on levels 0..L-1: pre-smooth (degree-2 Chebyshev from zero, one
 // stencil pass), residual, restriction, coarse correction, interpolation and
 // correction, post-smooth (degree-2 Chebyshev, two stencil passes).  Level L
@@ -17,11 +20,14 @@
 // the device: a CUDA graph with a conditional WHILE node.
 #include <cmath>
 #include <cstdlib>
+#include <algorithm>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include <cooperative_groups.h>
 
+#include "gb_direct_host.cuh"
 #include "gb_objects.cuh"
 #include "gb_tma.cuh"
 
@@ -717,12 +723,19 @@ struct gb_mixed {
     int nres = 0;     // partials written by the level-0 defect sweep
     cudaStream_t cap = nullptr;
     cudaGraphExec_t exec = nullptr;
+    // the direct correction (gb_direct.cu), where the level-0 operator is
+    // separable: its tables, and this solver as a group of one
+    DirectTables* dtab = nullptr;
+    DirectGroup* dgrp = nullptr;
+    const DirCtl* dres = nullptr;      // outcome of the last solve, if direct (pinned)
     ~gb_mixed() {
+        delete dgrp;
+        delete dtab;
         if (exec) cudaGraphExecDestroy(exec);
         if (cap) cudaStreamDestroy(cap);
         for (float* p : b) dfree(p);
         for (float* p : e) dfree(p);
-        for (float* p : t) dfree(p);
+        for (size_t l = 1; l < t.size(); l++) dfree(t[l]);   // t[0] lies in e[0]'s block
         dfree(direct_tab);
         dfree(coop_tab);
         dfree(tail_bar);
@@ -1358,8 +1371,16 @@ extern "C" int gb_mixed_new(int nlevels, gb_operator* op64, gb_operator* const* 
         const size_t bytes = (size_t)m->ops[l]->ng() * sizeof(float);
         float *bb = nullptr, *ee = nullptr, *tt = nullptr;
         ce = pool_malloc(&bb, bytes);
-        if (ce == cudaSuccess) ce = pool_malloc(&ee, bytes);
-        if (ce == cudaSuccess) ce = pool_malloc(&tt, bytes);
+        if (l == 0) {
+            // e and t of level 0 in one block, which is also the FP64 work
+            // grid of the direct path (a solve takes one path or the other)
+            const size_t half = (bytes + 255) / 256 * 256;
+            if (ce == cudaSuccess) ce = pool_malloc(&ee, 2 * half);
+            if (ce == cudaSuccess) tt = ee + half / sizeof(float);
+        } else {
+            if (ce == cudaSuccess) ce = pool_malloc(&ee, bytes);
+            if (ce == cudaSuccess) ce = pool_malloc(&tt, bytes);
+        }
         m->b.push_back(bb);
         m->e.push_back(ee);
         m->t.push_back(tt);
@@ -1475,8 +1496,81 @@ static int build_mixed_graph(gb_mixed* m) {
     return 0;
 }
 
+static int prepare_vcycles(gb_mixed* m);
+
+// --------------------------------------------------------- direct correction
+// Solves that allow at least this many V-cycles take the direct correction
+// where the grid has one.  V-cycle counts measured on every grid shape of
+// the benchmarks and tests are 10 to 23; a caller who allows fewer than 50
+// may be asking to be stopped, and is: such a solve keeps the V-cycles.
+constexpr int DIRECT_MIN_MAXITER = 50;
+
+static DirGrid direct_desc(const gb_mixed* m) {
+    DirGrid d{};
+    const GridBC& g = m->op64->g;
+    const CfdStencil& cs = m->op64->cs;
+    d.g = g;
+    double scale = fabs(cs.c0);
+    for (int a = 0; a < 3; a++) {
+        d.n[a] = g.n[a];
+        d.ax[a] = m->dtab->ax[a];
+        for (int k = 0; k < m->op64->nn; k++) {
+            d.cp[a][k] = cs.cp[a][k];
+            d.cm[a][k] = cs.cm[a][k];
+        }
+    }
+    d.c0 = cs.c0;
+    // the constant mode of a periodic grid: zero up to rounding; the next
+    // eigenvalue is at least (pi / n)^2 / 3 of the centre tap
+    d.tiny = 1e-12 * scale;
+    d.X = (double*)m->e[0];
+    return d;
+}
+
+static int build_direct_group(gb_mixed* m) {
+    m->dgrp = new DirectGroup();
+    if (int rc = m->dgrp->build({direct_desc(m)}, m->op64->nn, m->cap)) {
+        delete m->dgrp;
+        m->dgrp = nullptr;
+        return rc;
+    }
+    return 0;
+}
+
+extern "C" int gb_mixed_set_direct(gb_mixed* m, const double* const* pe, const double* const* po,
+                                   const double* const* lam) {
+    if (!m || !pe || !po || !lam) return fail(GB_EINVAL, "mixed direct: NULL argument");
+    if (m->dtab || m->exec) return fail(GB_EINVAL, "mixed direct: set it once, before a solve");
+    const GridBC& g = m->op64->g;
+    const CfdStencil& cs = m->op64->cs;
+    if (!pass_supported_grid(g, cs, m->op64->nn)) return 0;
+    for (int a = 0; a < 3; a++) {
+        const int he = g.periodic[a] ? g.n[a] / 2 + 1 : (g.n[a] + 1) / 2;
+        if (he > DIR_HMAX) return 0;
+        for (int k = 0; k < m->op64->nn; k++)
+            if (cs.cp[a][k] != cs.cm[a][k]) return 0;
+        if (!pe[a] || !lam[a] || (!po[a] && g.n[a] > he))
+            return fail(GB_EINVAL, "mixed direct: NULL table");
+    }
+    m->dtab = new DirectTables();
+    if (int rc = m->dtab->build(g, pe, po, lam)) {
+        delete m->dtab;
+        m->dtab = nullptr;
+        return rc;
+    }
+    return 0;
+}
+
 extern "C" int gb_mixed_prepare(gb_mixed* m) {
     if (!m) return fail(GB_EINVAL, "mixed prepare: NULL solver");
+    if (m->dtab) {
+        if (!m->dgrp) return build_direct_group(m);
+        return 0;
+    }
+    return prepare_vcycles(m);
+}
+
+static int prepare_vcycles(gb_mixed* m) {
     if (!m->exec) {
         int rc = build_mixed_graph(m);
         if (rc && m->coop) {
@@ -1496,9 +1590,23 @@ extern "C" int gb_mixed_solve_async(gb_mixed* m, double* phi, const double* rho,
     if (!m || !phi || !rho) return fail(GB_EINVAL, "mixed solve: NULL argument");
     if (maxiter < 1) return fail(GB_EINVAL, "mixed solve: maxiter must be >= 1");
     cudaStream_t st = (cudaStream_t)stream;
-    if (int rc = gb_mixed_prepare(m)) return rc;
     const long long n = m->op64->ng();
     const size_t bytes = (size_t)n * sizeof(double);
+    m->last_tol = tol;
+    m->last_maxiter = maxiter;
+    if (m->dtab && maxiter >= DIRECT_MIN_MAXITER) {
+        if (!m->dgrp)
+            if (int rc = build_direct_group(m)) return rc;
+        m->dres = m->dgrp->ctl_host;
+        if (ranges_overlap(phi, rho, bytes)) {
+            // phi changes while rho is still read: a copy of rho
+            GB_CUDA_TRY(cudaMemcpyAsync(m->rho0, rho, bytes, cudaMemcpyDeviceToDevice, st));
+            rho = m->rho0;
+        }
+        return m->dgrp->solve(phi, rho, tol, maxiter, st);
+    }
+    m->dres = nullptr;
+    if (int rc = prepare_vcycles(m)) return rc;
     GB_CUDA_TRY(cudaMemcpyAsync(m->rho0, rho, bytes, cudaMemcpyDeviceToDevice, st));
     GB_CUDA_TRY(cudaMemcpyAsync(m->phi0, phi, bytes, cudaMemcpyDeviceToDevice, st));
     const int nb = (int)std::min<long long>(1024, (n + 255) / 256);
@@ -1509,13 +1617,15 @@ extern "C" int gb_mixed_solve_async(gb_mixed* m, double* phi, const double* rho,
     GB_CUDA_TRY(cudaGraphLaunch(m->exec, st));
     GB_CUDA_TRY(cudaMemcpyAsync(phi, m->phi0, bytes, cudaMemcpyDeviceToDevice, st));
     GB_CUDA_TRY(cudaMemcpyAsync(m->ctl_host, m->ctl, sizeof(Ctl), cudaMemcpyDeviceToHost, st));
-    m->last_tol = tol;
-    m->last_maxiter = maxiter;
     return 0;
 }
 
 extern "C" int gb_mixed_result(gb_mixed* m, int* niter, double* rel_residual) {
     if (!m) return fail(GB_EINVAL, "mixed result: NULL solver");
+    if (m->dres) {
+        m->ctl_host->niter = m->dres->niter;
+        m->ctl_host->rel = m->dres->rel;
+    }
     if (niter) *niter = m->ctl_host->niter;
     if (rel_residual) *rel_residual = m->ctl_host->rel;
     if (m->ctl_host->rel > m->last_tol)
@@ -1568,7 +1678,15 @@ struct gb_mixed_batch {
     long long* d_len = nullptr;    // [n] points of grid i
     cudaStream_t cap = nullptr;
     cudaGraphExec_t exec = nullptr;
+    DirectGroup* dgrp = nullptr;   // every grid by the direct correction
     ~gb_mixed_batch() {
+        for (int i = 0; i < n && dgrp; i++)     // results outlive the batch
+            if (s[i]->dres == dgrp->ctl_host + i) {
+                s[i]->ctl_host->niter = s[i]->dres->niter;
+                s[i]->ctl_host->rel = s[i]->dres->rel;
+                s[i]->dres = nullptr;
+            }
+        delete dgrp;
         if (exec) cudaGraphExecDestroy(exec);
         if (cap) cudaStreamDestroy(cap);
         cudaFree(d_user);
@@ -1658,6 +1776,35 @@ int add_branch(gb_mixed_batch* bt, cudaGraph_t G, gb_mixed* m, cudaGraphNode_t r
     return 0;
 }
 
+// does any phi of this launch share memory with any rho?
+bool batch_overlaps(const gb_mixed_batch* bt) {
+    std::vector<std::pair<const char*, const char*>> r(bt->n);
+    for (int i = 0; i < bt->n; i++) {
+        const char* a = (const char*)bt->h_user[2 * i + 1];
+        r[i] = {a, a + bt->s[i]->op64->ng() * sizeof(double)};
+    }
+    std::sort(r.begin(), r.end());
+    for (int i = 1; i < bt->n; i++) r[i].second = std::max(r[i].second, r[i - 1].second);
+    for (int i = 0; i < bt->n; i++) {
+        const char* a = (const char*)bt->h_user[2 * i];
+        const char* b = a + bt->s[i]->op64->ng() * sizeof(double);
+        // the rhos that start below b, and the largest end among them
+        auto it = std::lower_bound(r.begin(), r.end(), std::make_pair(b, (const char*)nullptr));
+        if (it != r.begin() && std::prev(it)->second > a) return true;
+    }
+    return false;
+}
+
+int build_direct_batch(gb_mixed_batch* bt) {
+    const int n = bt->n;
+    std::vector<DirGrid> d;
+    for (gb_mixed* m : bt->s) d.push_back(direct_desc(m));
+    GB_CUDA_TRY(cudaMalloc(&bt->d_user, 2 * n * sizeof(double*)));
+    GB_CUDA_TRY(cudaMallocHost(&bt->h_user, 2 * n * sizeof(double*)));
+    bt->dgrp = new DirectGroup();
+    return bt->dgrp->build(d, bt->s[0]->op64->nn, bt->cap);
+}
+
 int build_batch(gb_mixed_batch* bt) {
     const int n = bt->n;
     long long maxlen = 0;
@@ -1730,10 +1877,16 @@ extern "C" int gb_mixed_batch_new(int n, gb_mixed* const* solvers, double tol, i
         for (int j = 0; j < i; j++)
             if (solvers[j] == solvers[i])
                 return fail(GB_EINVAL, "mixed batch: solver %d appears twice", i);
-        // one uncaptured pass of every kernel (sets kernel attributes)
+    }
+    // the direct path when every grid has one (and the same half-width, which
+    // the grouped defect kernel is compiled for)
+    bool direct = maxiter >= DIRECT_MIN_MAXITER;
+    for (int i = 0; i < n; i++)
+        direct = direct && solvers[i]->dtab && solvers[i]->op64->nn == solvers[0]->op64->nn;
+    // one uncaptured pass of every kernel (sets kernel attributes)
+    for (int i = 0; i < n && !direct; i++)
         if (!solvers[i]->exec)
             if (int rc = build_mixed_graph(solvers[i])) return rc;
-    }
     gb_mixed_batch* bt = new gb_mixed_batch();
     bt->tol = tol;
     bt->maxiter = maxiter;
@@ -1744,7 +1897,7 @@ extern "C" int gb_mixed_batch_new(int n, gb_mixed* const* solvers, double tol, i
         delete bt;
         return fail(GB_ECUDA, "mixed batch: stream: %s", cudaGetErrorString(e));
     }
-    if (int rc = build_batch(bt)) {
+    if (int rc = direct ? build_direct_batch(bt) : build_batch(bt)) {
         delete bt;
         return rc;
     }
@@ -1766,9 +1919,20 @@ extern "C" int gb_mixed_batch_solve_async(gb_mixed_batch* bt, double* const* phi
         bt->h_user[2 * i + 1] = const_cast<double*>(rhos[i]);
         bt->s[i]->last_tol = bt->tol;
         bt->s[i]->last_maxiter = bt->maxiter;
+        bt->s[i]->dres = bt->dgrp ? bt->dgrp->ctl_host + i : nullptr;
     }
+    if (bt->dgrp && batch_overlaps(bt))
+        // some phi changes while a rho that it shares memory with is still
+        // read: copies of every rho
+        for (int i = 0; i < bt->n; i++) {
+            gb_mixed* m = bt->s[i];
+            GB_CUDA_TRY(cudaMemcpyAsync(m->rho0, rhos[i], m->op64->ng() * sizeof(double),
+                                        cudaMemcpyDeviceToDevice, st));
+            bt->h_user[2 * i + 1] = m->rho0;
+        }
     GB_CUDA_TRY(cudaMemcpyAsync(bt->d_user, bt->h_user, 2 * bt->n * sizeof(double*),
                                 cudaMemcpyHostToDevice, st));
+    if (bt->dgrp) return bt->dgrp->solve_batch(bt->d_user, bt->tol, bt->maxiter, st);
     GB_CUDA_TRY(cudaGraphLaunch(bt->exec, st));
     return 0;
 }
@@ -1777,7 +1941,11 @@ extern "C" int gb_mixed_batch_result(gb_mixed_batch* bt, int* niters, double* re
     if (!bt) return fail(GB_EINVAL, "mixed batch result: NULL batch");
     int bad = -1;
     for (int i = 0; i < bt->n; i++) {
-        const Ctl* c = bt->s[i]->ctl_host;
+        Ctl* c = bt->s[i]->ctl_host;
+        if (bt->dgrp) {
+            c->niter = bt->dgrp->ctl_host[i].niter;
+            c->rel = bt->dgrp->ctl_host[i].rel;
+        }
         if (niters) niters[i] = c->niter;
         if (rel_residuals) rel_residuals[i] = c->rel;
         if (c->rel > bt->tol && bad < 0) bad = i;

@@ -20,6 +20,7 @@
 // instruction.  Rows of the solver's arrays are not 16-byte aligned (odd
 // sides), which rules out TMA here; the shared-memory tile is aligned
 // instead.
+#include "gb_direct.cuh"
 #include "gb_objects.cuh"
 
 namespace gb {
@@ -54,7 +55,10 @@ enum : int {
     // double only: the preconditioner step out = +-(u - sc (A u - aux)) with
     // the stencil summed and every product and sum rounded as the
     // reference's C loop does (bit-identical); p0 = sc, p1 != 0 negates
-    PF_EXACT_PRECOND = 32
+    PF_EXACT_PRECOND = 32,
+    // double only, with PF_PARTIAL: each CTA also writes the partial sum of
+    // aux^2, the two interleaved
+    PF_AUXSQ = 64
 };
 
 template <class T>
@@ -89,12 +93,14 @@ constexpr int pass_min_blocks() {
     return (F & PF_ACC64) ? 2 : 3;
 }
 
+// the pass of one CTA: tile bx of the planes [by chunk, ...) of grid bz;
+// partial sums go to slot by * nbx + bx
 template <class T, int NN, int F>
-__global__ void __launch_bounds__(256, pass_min_blocks<F>())
-k_pass(const T* __restrict__ u, T* __restrict__ out, const T* __restrict__ aux,
-       const T* __restrict__ aux2, double* __restrict__ acc64, float* __restrict__ out32,
-       double* __restrict__ partial, GridBC g, PassCoef<T> c, T p0, T p1, T p2, T p3, int chunk,
-       int tiles_x) {
+__device__ __forceinline__ void
+pass_body(const T* __restrict__ u, T* __restrict__ out, const T* __restrict__ aux,
+          const T* __restrict__ aux2, double* __restrict__ acc64, float* __restrict__ out32,
+          double* __restrict__ partial, const GridBC& g, const PassCoef<T>& c, T p0, T p1, T p2,
+          T p3, int chunk, int tiles_x, int bx, int by, int bz, int nbx) {
     constexpr int VX = PassVec<T>::N;
     constexpr int TX = 16 * VX;
     constexpr int C = TX + 2 * PT_HX;           // staged columns
@@ -113,12 +119,12 @@ k_pass(const T* __restrict__ u, T* __restrict__ out, const T* __restrict__ aux,
     const long long ps = (long long)n1 * n2;
     const int tid = threadIdx.x;
     const int tx = tid & 15, ty = tid >> 4;
-    const int x0 = (blockIdx.x % tiles_x) * TX, y0 = (blockIdx.x / tiles_x) * PT_ROWS;
+    const int x0 = (bx % tiles_x) * TX, y0 = (bx / tiles_x) * PT_ROWS;
     const int x = x0 + VX * tx, y = y0 + ty;
-    const int pa = blockIdx.y * chunk;
+    const int pa = by * chunk;
     const int pb = min(n0, pa + chunk);
-    {   // grid blockIdx.z of a batch
-        const long long off = (long long)blockIdx.z * n0 * ps;
+    {   // grid bz of a batch
+        const long long off = (long long)bz * n0 * ps;
         u += off;
         if (out) out += off;
         if (aux) aux += off;
@@ -206,7 +212,7 @@ k_pass(const T* __restrict__ u, T* __restrict__ out, const T* __restrict__ aux,
         }
     };
     load_pointwise(pa);
-    double sq = 0.0;
+    double sq = 0.0, sq2 = 0.0;
     const int col0 = PT_HX + VX * tx;
     for (int p = pa; p < pb; p++) {
         T ca[VX], cb[VX];
@@ -312,6 +318,7 @@ k_pass(const T* __restrict__ u, T* __restrict__ out, const T* __restrict__ aux,
                 if (F & PF_AUX) v = fma(p0, ca[j], v);
                 if (F & PF_AUX2) v = fma(p3, cb[j], v);
                 if (F & PF_PARTIAL) sq = fma((double)v, (double)v, sq);
+                if (F & PF_AUXSQ) sq2 = fma((double)ca[j], (double)ca[j], sq2);
                 if (F & PF_ACC64)
                     acc64[row + j] = cc[j] + (double)v;
                 else if (F & PF_OUT32)
@@ -322,10 +329,51 @@ k_pass(const T* __restrict__ u, T* __restrict__ out, const T* __restrict__ aux,
         }
     }
     asm volatile("cp.async.wait_group 0;\n" ::);
-    if (F & PF_PARTIAL) {
+    if (F & PF_AUXSQ) {
+        const double s = block_sum(sq), s2 = block_sum(sq2);
+        if (tid == 0) {
+            partial[2 * (by * nbx + bx)] = s;
+            partial[2 * (by * nbx + bx) + 1] = s2;
+        }
+    } else if (F & PF_PARTIAL) {
         const double s = block_sum(sq);
-        if (tid == 0) partial[blockIdx.y * gridDim.x + blockIdx.x] = s;
+        if (tid == 0) partial[by * nbx + bx] = s;
     }
+}
+
+template <class T, int NN, int F>
+__global__ void __launch_bounds__(256, pass_min_blocks<F>())
+k_pass(const T* __restrict__ u, T* __restrict__ out, const T* __restrict__ aux,
+       const T* __restrict__ aux2, double* __restrict__ acc64, float* __restrict__ out32,
+       double* __restrict__ partial, GridBC g, PassCoef<T> c, T p0, T p1, T p2, T p3, int chunk,
+       int tiles_x) {
+    pass_body<T, NN, F>(u, out, aux, aux2, acc64, out32, partial, g, c, p0, p1, p2, p3, chunk,
+                        tiles_x, blockIdx.x, blockIdx.y, blockIdx.z, gridDim.x);
+}
+
+// The FP64 defect X = rho - L phi of a group of grids (a batch of the mixed
+// solver's direct path) in one launch, with partial sums of d^2 and rho^2.
+template <int NN>
+__global__ void __launch_bounds__(256, 3)
+k_defect_group(const DirGrid* __restrict__ grids, const DirCtl* ctl,
+               const DirBlock* __restrict__ map) {
+    DirBlock bk{0, (int)blockIdx.x};
+    if (map) bk = map[blockIdx.x];
+    if (!ctl[bk.grid].active) return;
+    const DirGrid& G = grids[bk.grid];
+    const GridBC g = G.g;
+    PassCoef<double> c;
+    c.c0 = G.c0;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+#pragma unroll
+        for (int d = 0; d < 3; d++) {
+            c.cp[k][d] = G.cp[k][d];
+            c.cm[k][d] = G.cm[k][d];
+        }
+    pass_body<double, NN, PF_AUX | PF_PARTIAL | PF_AUXSQ>(
+        G.phi, G.X, G.rho, nullptr, nullptr, nullptr, G.partial, g, c, 1.0, 0.0, -1.0, 0.0,
+        G.chunk, G.tiles_x, bk.block % G.tiles, bk.block / G.tiles, 0, G.tiles);
 }
 
 
@@ -437,6 +485,37 @@ int launch_pass(const GridBC& g, const CfdStencil& cs, int nn, const T* in, T* o
         case 2: return launch_pass_nn<T, 2>(f, g, c, in, out, aux, aux2, acc64, out32, partial, a0, a1, a2, a3, st);
         default: return launch_pass_nn<T, 3>(f, g, c, in, out, aux, aux2, acc64, out32, partial, a0, a1, a2, a3, st);
     }
+}
+
+int launch_defect_group(int nn, const DirGrid* grids, const DirCtl* ctl, const DirBlock* map,
+                        int nblocks, cudaStream_t st) {
+    const size_t smem = (size_t)PT_RING * (PT_ROWS + 2 * nn) *
+                        (16 * PassVec<double>::N + 2 * PT_HX) * sizeof(double);
+    auto go = [&](auto kernel) {
+        // (set on every call: cheap, and safe from several threads)
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem) != cudaSuccess)
+            return -2;
+        kernel<<<nblocks, 256, smem, st>>>(grids, ctl, map);
+        return 0;
+    };
+    switch (nn) {
+        case 1: return go(k_defect_group<1>);
+        case 2: return go(k_defect_group<2>);
+        case 3: return go(k_defect_group<3>);
+    }
+    return -1;
+}
+
+void defect_group_geom(const GridBC& g, int per_grid_blocks, int& chunk, int& tiles_x, int& tiles,
+                       int& nblk) {
+    constexpr int TX = 16 * PassVec<double>::N;
+    tiles_x = (g.n[2] + TX - 1) / TX;
+    tiles = tiles_x * ((g.n[1] + PT_ROWS - 1) / PT_ROWS);
+    // at least 8 planes a CTA: a chunk reads 2 nn planes of its neighbours
+    const int want = std::max(1, std::min(per_grid_blocks / tiles, (g.n[0] + 7) / 8));
+    chunk = (g.n[0] + want - 1) / want;
+    nblk = tiles * ((g.n[0] + chunk - 1) / chunk);
 }
 
 int launch_pass_precond(const GridBC& g, const CfdStencil& cs, int nn, const double* in,

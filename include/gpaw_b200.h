@@ -322,6 +322,22 @@ GB_API void gb_mixed_free(gb_mixed* m);
  * different FP32 corrections, each deterministic.  No counterpart in the
  * reference.  Returns 0; a mode the levels do not allow falls back to 0. */
 GB_API int gb_mixed_set_fused_coarse(gb_mixed* m, int mode);
+/* Give the solver its direct correction: the eigenvectors of the level-0
+ * operator's one-dimensional parts.  Along axis a (n points) the halves that
+ * are even and odd under the reflection j <-> n - 1 - j (zero boundary) or
+ * j <-> (n - j) mod n (periodic): pe[a] is h x h row-major [point][mode] with
+ * h = (n + 1) / 2 (zero) or n / 2 + 1 (periodic) for the points 0 .. h - 1,
+ * po[a] the same for the n - h points that have a distinct mirror point;
+ * columns of unit norm over all n points.  lam[a]: n eigenvalues, even first;
+ * their sum over the axes is the operator's eigenvalue.  Solves that allow at least 50
+ * V-cycles then correct phi by e = L^-1 d in FP64 (fast diagonalisation)
+ * instead of an FP32 V-cycle, inside the same defect-correction loop;
+ * V-cycle counts become counts of corrections (one or two).  A grid the path
+ * does not take (stencils wider than 3, more than 384 points a side,
+ * unsymmetric coefficients) keeps the V-cycles; returns 0 either way.  Call
+ * it once, before the first solve.  No counterpart in the reference. */
+GB_API int gb_mixed_set_direct(gb_mixed* m, const double* const* pe, const double* const* po,
+                               const double* const* lam);
 /* One V-cycle of the mixed-precision solver and the defects around it,
  * launched kernel by kernel instead of through the solver's graph:
  * phi <- phi + V32(rho - L phi).  For profilers and kernel traces (its
@@ -356,9 +372,11 @@ GB_API int gb_mixed_result(gb_mixed* m, int* niter, double* rel_residual);
 GB_API int gb_mixed_prepare(gb_mixed* m);
 
 /* Many mixed-precision solves as one CUDA graph (no reference counterpart):
- * one branch per solver (distinct solvers, grids of any sizes), each the
- * solve of gb_mixed_solve_async with tolerance `tol` and at most `maxiter`
- * V-cycles; the branches run concurrently.  gb_mixed_batch_solve_async
+ * distinct solvers, grids of any sizes, each the solve of
+ * gb_mixed_solve_async with tolerance `tol` and at most `maxiter`
+ * corrections: by grouped kernels over all grids when every solver has the
+ * direct correction (and maxiter allows it), else one branch of V-cycles per
+ * solver, the branches side by side.  gb_mixed_batch_solve_async
  * takes one phi and one rho per solver (device arrays of that solver's
  * grid), enqueues the whole batch with one graph launch and returns;
  * gb_mixed_batch_result (after the stream reached that point) fills

@@ -205,6 +205,12 @@ extern "C" int gb_operator_new(const double* coefs, const int64_t* offsets, int 
     const char* path = getenv("GPAW_B200_FD_PATH");
     const bool force_generic = path && strcmp(path, "generic") == 0;
     op->tiled = (!force_generic && to_cfd_stencil(op->st, op->cs, op->nn)) ? 1 : 0;
+    bool axis_aligned = true;
+    for (int p = 0; p < ncoefs; p++) {
+        const int* o = op->st.off[p];
+        axis_aligned = axis_aligned && (o[0] != 0) + (o[1] != 0) + (o[2] != 0) <= 1;
+    }
+    op->general = range <= 6 && (!cfd || axis_aligned);
     *out = op;
     return 0;
 }

@@ -113,6 +113,7 @@ struct gb_operator {
     gb::CfdStencil cs;     // axis-aligned form, when the stencil has one
     int nn = 0;        // its half-width
     int tiled = 0;     // use the plane-marching kernels
+    int general = 0;   // otherwise: the tiled kernel for general stencils takes it
     int chunk = 0;     // axis-0 planes per CTA of those kernels (0: automatic)
     gb::Scratch scratch;   // aliasing stage / Jacobi ping-pong / GS snapshot
     gb::Scratch partial;   // per-CTA partial sums of |r|^2
@@ -133,7 +134,8 @@ namespace gb {
 
 // Partial sums produced per grid by a residual sweep of `op`.
 inline int op_resid_blocks(const gb_operator* op, int nin, int es) {
-    return op->tiled ? cfd_blocks(op->g, op->nn, es, nin, op->chunk) : residual_blocks(op->g);
+    return op->tiled ? cfd_blocks(op->g, op->nn, es, nin, op->chunk) 
+           : op->general ? general_blocks(op->g, op->st.range, nin, es) : residual_blocks(op->g);
 }
 
 // One pass of the stencil with a fused epilogue; plane-marching kernel for
@@ -152,6 +154,16 @@ inline int op_sweep(gb_operator* op, int mode, const void* in, void* out, const 
         if (rc == -2) return fail(GB_ECUDA, "could not raise the shared-memory limit");
         if (rc == 0) return 0;
     }
+    if (op->general) {
+        const Epi ep{aux, w, sc, negate, partial};
+        const int rc = dtype == GB_F64
+                           ? launch_general<double>(mode, in, out, nin, op->g, P, op->st, ep, st)
+                           : launch_general<double2>(mode, in, out, nin, op->g, P, op->st, ep, st);
+        if (rc == -2) return fail(GB_ECUDA, "could not raise the shared-memory limit");
+        if (rc == 0) return 0;
+    }
+    // one thread a point: ranges above 6, and diagonal taps declared
+    // axis-aligned (whose corner values read zero)
     switch (mode) {
         case EPI_APPLY:
             if (dtype == GB_F64) launch_fd<double>(in, out, nin, op->g, P, op->st, st);

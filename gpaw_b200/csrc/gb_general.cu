@@ -7,37 +7,44 @@
 // every product and sum rounded on its own.
 //
 // 24 x 72 x 72 x 100 complex, hexagonal, nn = 3: 613 us one thread a point
-// through L1 (every warp straddled a periodic edge), 323 us here.
+// through L1 (every warp straddled a periodic edge), 323 us with fixed 32 x 16
+// tiles, 274 us with tiles that divide the plane evenly.
 //
 // What bounds it: every tap is one shared-memory read (16 bytes a complex
 // point: 25 taps of a hexagonal cell's nn = 3 Laplacian take 3.1 clocks of an
 // SM a point, against 1.4 for its HBM traffic), so the other work of a tap
-// has to be small.  A CTA owns a 32 x 16 column tile and a chunk of planes
-// along axis 0; planes with their halo (corners too) stream by cp.async into
-// a ring of 2 R + 2 stages.  A thread owns two points eight rows apart, so a
+// has to be small.  A CTA owns a column tile of up to 512 points (its sides
+// divide the plane evenly) and a chunk of planes along axis 0; planes with their halo (corners too) stream by cp.async into
+// a ring of 2 R + 2 stages.  A thread owns two points of the tile, so a
 // tap's address (its byte offset from a kernel parameter, wrapped at the
 // ring's end by one unsigned minimum) serves both.  Wrap-around is folded
 // into the copy's source, and Bloch phases are applied once a cell, right
 // after it lands, axis by axis as the reference fills its halo
 // (c/bc.cpp:108-112, 242-257).
 #include <algorithm>
+#include <type_traits>
 
 #include "gb_objects.cuh"
+#include "gb_split.cuh"
 
 namespace gb {
 namespace {
 
-constexpr int GY = 16;
-// tile columns: 16 where the ring of 32-wide tiles would not fit an SM
+constexpr int GT = 256;         // threads; two points each
+// CTAs an SM, and the cells of a staged plane that this leaves room for
 template <class T, int R>
-constexpr int gen_gx() {
-    return (2 * R + 2) * (32 + 2 * R) * (GY + 2 * R) * (int)sizeof(T) <= 227 * 1024 ? 32 : 16;
+constexpr int gen_blocks() {
+    return sizeof(T) == 16 ? (R <= 3 ? 2 : 1) : (R <= 4 ? 3 : 2);
+}
+template <class T, int R>
+constexpr int gen_cells() {
+    const int fit = (226 * 1024 / gen_blocks<T, R>() - 1024) / ((2 * R + 2) * (int)sizeof(T));
+    return fit < 1536 ? fit : 1536;
 }
 
 // a stencil as byte offsets into the ring
 struct Taps {
     int n;
-    int range;
     double coef[GB_MAX_COEFS];
     unsigned off[GB_MAX_COEFS];    // stage offset (mod the ring) + in-plane offset
 };
@@ -62,22 +69,24 @@ __device__ __forceinline__ bool into(int& y, int n, int periodic) {
 
 // R: the stencil's range, at most this; MODE as in gb_internal.cuh
 template <class T, int R, int MODE>
-__global__ void __launch_bounds__(8 * gen_gx<T, R>(), sizeof(T) == 16 ? (R <= 3 ? 2 : 1) : (R <= 4 ? 3 : 2))
+__global__ void __launch_bounds__(GT, gen_blocks<T, R>())
 k_general(const T* __restrict__ in, T* __restrict__ out, GridBC g, Phases P,
-          const __grid_constant__ Taps s, int chunk, int tiles_x, Epi ep) {
+          const __grid_constant__ Taps s, int chunk, int tiles_x, int tw, int th, Epi ep) {
     constexpr bool CPLX = sizeof(T) == 16;
-    constexpr int GX = gen_gx<T, R>(), GT = 8 * GX;
-    constexpr int PX = GX + 2 * R, PY = GY + 2 * R, E = PX * PY, S = 2 * R + 2;
-    constexpr unsigned EB = sizeof(T), PB = E * EB, RING = S * PB;
-    constexpr int NC = (E + GT - 1) / GT;
+    constexpr int S = 2 * R + 2, NC = (gen_cells<T, R>() + GT - 1) / GT;
+    constexpr unsigned EB = sizeof(T);
+    const int PX = tw + 2 * R, E = PX * (th + 2 * R);
+    const unsigned PB = E * EB, RING = S * PB;
     extern __shared__ __align__(16) unsigned char gen_smem[];
     const unsigned ring = (unsigned)__cvta_generic_to_shared(gen_smem);
 
     const int n0 = g.n[0], n1 = g.n[1], n2 = g.n[2];
     const long long ps = (long long)n1 * n2, grid0 = (long long)blockIdx.z * n0 * ps;
-    const int tid = threadIdx.x, tx = tid % GX, ty = tid / GX;
-    const int x0 = (blockIdx.x % tiles_x) * GX, y0 = (blockIdx.x / tiles_x) * GY;
-    const int x = x0 + tx, y = y0 + ty;
+    const int tid = threadIdx.x;
+    const int x0 = (blockIdx.x % tiles_x) * tw, y0 = (blockIdx.x / tiles_x) * th;
+    // this thread's points: number tid and tid + 256 of the tile, row by row
+    const int ra = min(tid / tw, th - 1), ca_ = tid % tw;
+    const int rb = min((tid + GT) / tw, th - 1), cb_ = (tid + GT) % tw;
     const int pa = blockIdx.y * chunk, pb = min(n0, pa + chunk);
     const T* a = in + grid0;
 
@@ -133,13 +142,15 @@ k_general(const T* __restrict__ in, T* __restrict__ out, GridBC g, Phases P,
         }
     };
 
-    const bool live0 = x < n2 && y < n1, live1 = x < n2 && y + 8 < n1;
-    const long long at0 = (long long)y * n2 + x;
+    const bool live0 = tid < tw * th && x0 + ca_ < n2 && y0 + ra < n1;
+    const bool live1 = tid + GT < tw * th && x0 + cb_ < n2 && y0 + rb < n1;
+    const long long at0 = (long long)(y0 + ra) * n2 + x0 + ca_;
     constexpr bool AUX = MODE != EPI_APPLY;
     const T* aux = !AUX || MODE == EPI_POT ? nullptr : (const T*)ep.aux + grid0 + at0;
     const double* pot = MODE == EPI_POT ? (const double*)ep.aux + at0 : nullptr;
     T* o = out ? out + grid0 + at0 : nullptr;
-    const long long row8 = 8ll * n2;
+    const long long second = (long long)(rb - ra) * n2 + cb_ - ca_;   // second point
+    const int delta = ((rb - ra) * PX + cb_ - ca_) * (int)EB;
     double sq = 0.0;
 
     // planes pa - R .. pa + R, all landed but the last
@@ -155,10 +166,10 @@ k_general(const T* __restrict__ in, T* __restrict__ out, GridBC g, Phases P,
             const long long q = p * ps;
             if constexpr (MODE == EPI_POT) {
                 if (live0) cp0 = pot[q];
-                if (live1) cp1 = pot[q + row8];
+                if (live1) cp1 = pot[q + second];
             } else {
                 if (live0) ca0 = aux[q];
-                if (live1) ca1 = aux[q + row8];
+                if (live1) ca1 = aux[q + second];
             }
         }
         int front = slot + R;
@@ -170,12 +181,12 @@ k_general(const T* __restrict__ in, T* __restrict__ out, GridBC g, Phases P,
         issue(p + R + 1, front + 1 == S ? 0 : front + 1);
         // byte address of the first point relative to the ring, one ring up
         // for the offsets that point back
-        const unsigned cen = slot * PB + ((ty + R) * PX + tx + R) * EB;
+        const unsigned cen = slot * PB + ((ra + R) * PX + ca_ + R) * EB;
         T xa = Num<T>::zero(), xb = Num<T>::zero(), va, vb;
         auto read = [&](unsigned at, T& u, T& v) {
             const unsigned char* b = gen_smem + at;
             u = *reinterpret_cast<const T*>(b);
-            v = *reinterpret_cast<const T*>(b + 8 * PX * EB);
+            v = *reinterpret_cast<const T*>(b + delta);
         };
         read(cen, va, vb);
 #pragma unroll 6
@@ -210,7 +221,7 @@ k_general(const T* __restrict__ in, T* __restrict__ out, GridBC g, Phases P,
         }
         if (MODE != EPI_RESID || out) {
             if (live0) o[p * ps] = xa;
-            if (live1) o[p * ps + row8] = xb;
+            if (live1) o[p * ps + second] = xb;
         }
         slot = slot + 1 == S ? 0 : slot + 1;
     }
@@ -224,26 +235,36 @@ k_general(const T* __restrict__ in, T* __restrict__ out, GridBC g, Phases P,
 }
 
 struct Geom {
-    int tiles_x, tiles, chunk, nchunk;
+    int tw, th, tiles_x, tiles, chunk, nchunk;
 };
 
-// Chunk of planes a CTA marches through: the split of axis 0 with the least
-// waves x (planes + the 2 R it reads before the first), two CTAs an SM.
-Geom geom(const GridBC& g, int R, int nin, int GX) {
-    Geom G;
-    G.tiles_x = (g.n[2] + GX - 1) / GX;
-    G.tiles = G.tiles_x * ((g.n[1] + GY - 1) / GY);
+// Tile: the even split of the plane into tw x th pieces of at most 512 points
+// (two a thread) whose staged plane fits, with the least work: a tap reads
+// shared memory for all 512 points, a staged cell is written once.  (A fixed
+// 32 x 16 tile computes 1.42 times the points of a 72 x 100 plane.)  Chunk of
+// axis 0: least waves x planes.
+Geom geom(const GridBC& g, int R, int ncoefs, int nin, int cells, int blocks) {
+    Geom G{};
     long long best = -1;
-    for (int k = 1; k <= g.n[0]; k++) {
-        const int chunk = (g.n[0] + k - 1) / k;
-        const long long ctas = (long long)G.tiles * nin * ((g.n[0] + chunk - 1) / chunk);
-        const long long cost = (ctas + 295) / 296 * (chunk + 2 * R);
+    for (int kx = 1; kx <= g.n[2]; kx++) {
+        const int tw = (g.n[2] + kx - 1) / kx;
+        if (tw > 512) continue;
+        int th = std::min(512 / tw, cells / (tw + 2 * R) - 2 * R);
+        if (th < 1) continue;
+        const int ky = (g.n[1] + th - 1) / th;
+        th = (g.n[1] + ky - 1) / ky;
+        const long long cost = (long long)((g.n[2] + tw - 1) / tw) * ky *
+                               (512ll * ncoefs + 2ll * (tw + 2 * R) * (th + 2 * R));
         if (best < 0 || cost < best) {
             best = cost;
-            G.chunk = chunk;
+            G.tw = tw;
+            G.th = th;
         }
-        if (ctas >= 8 * 296 && k > 1) break;
+        if (tw <= 8) break;
     }
+    G.tiles_x = (g.n[2] + G.tw - 1) / G.tw;
+    G.tiles = G.tiles_x * ((g.n[1] + G.th - 1) / G.th);
+    G.chunk = split_planes(g.n[0], 1, 2 * R, (long long)G.tiles * nin, 148 * blocks);
     G.nchunk = (g.n[0] + G.chunk - 1) / G.chunk;
     return G;
 }
@@ -251,21 +272,20 @@ Geom geom(const GridBC& g, int R, int nin, int GX) {
 template <class T, int R, int MODE>
 int launch_r(const void* in, void* out, int nin, const GridBC& g, const Phases& P,
              const Stencil& st, const Epi& ep, cudaStream_t stream) {
-    constexpr int GX = gen_gx<T, R>(), GT = 8 * GX;
-    constexpr int PX = GX + 2 * R, E = PX * (GY + 2 * R), S = 2 * R + 2;
-    constexpr int smem = S * E * (int)sizeof(T);
+    constexpr int S = 2 * R + 2;
+    const Geom G = geom(g, R, st.ncoefs, nin, gen_cells<T, R>(), gen_blocks<T, R>());
+    const int PX = G.tw + 2 * R, E = PX * (G.th + 2 * R);
+    const int smem = S * E * (int)sizeof(T);
     if (cudaFuncSetAttribute(k_general<T, R, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              smem) != cudaSuccess)
         return -2;
     Taps s;
     s.n = st.ncoefs;
-    s.range = st.range;
     for (int c = 0; c < st.ncoefs; c++) {
         s.coef[c] = st.coef[c];
         const int stage = st.off[c][0] < 0 ? st.off[c][0] + S : st.off[c][0];
         s.off[c] = (unsigned)((stage * E + st.off[c][1] * PX + st.off[c][2]) * (int)sizeof(T));
     }
-    const Geom G = geom(g, R, nin, GX);
     const long long ng = (long long)g.n[0] * g.n[1] * g.n[2];
     for (int b0 = 0; b0 < nin; b0 += 65535) {
         const int nb = std::min(65535, nin - b0);
@@ -274,7 +294,7 @@ int launch_r(const void* in, void* out, int nin, const GridBC& g, const Phases& 
         if (e.partial) e.partial = ep.partial + (long long)b0 * G.tiles * G.nchunk;
         k_general<T, R, MODE><<<dim3(G.tiles, G.nchunk, nb), GT, smem, stream>>>(
             (const T*)in + b0 * ng, out ? (T*)out + b0 * ng : nullptr, g, P, s, G.chunk,
-            G.tiles_x, e);
+            G.tiles_x, G.tw, G.th, e);
     }
     return 0;
 }
@@ -293,8 +313,6 @@ int launch_m(const void* in, void* out, int nin, const GridBC& g, const Phases& 
     }
     return -1;
 }
-
-static_assert(gen_gx<double2, 5>() == 32 && gen_gx<double, 6>() == 32, "general_blocks");
 
 }  // namespace
 
@@ -318,10 +336,26 @@ template int launch_general<double>(int, const void*, void*, int, const GridBC&,
 template int launch_general<double2>(int, const void*, void*, int, const GridBC&, const Phases&,
                                      const Stencil&, const Epi&, cudaStream_t);
 
-int general_blocks(const GridBC& g, int range, int nin, int elem_bytes) {
-    const Geom G = geom(g, std::max(1, range), nin,
-                        elem_bytes == 16 && range == 6 ? gen_gx<double2, 6>() : 32);
-    return G.tiles * G.nchunk;
+template <class T>
+static int blocks_of(const GridBC& g, int range, int ncoefs, int nin) {
+    auto of = [&](auto R_) {
+        constexpr int R = decltype(R_)::value;
+        const Geom G = geom(g, R, ncoefs, nin, gen_cells<T, R>(), gen_blocks<T, R>());
+        return G.tiles * G.nchunk;
+    };
+    switch (range) {
+        case 2: return of(std::integral_constant<int, 2>{});
+        case 3: return of(std::integral_constant<int, 3>{});
+        case 4: return of(std::integral_constant<int, 4>{});
+        case 5: return of(std::integral_constant<int, 5>{});
+        case 6: return of(std::integral_constant<int, 6>{});
+    }
+    return of(std::integral_constant<int, 1>{});
+}
+
+int general_blocks(const GridBC& g, int range, int ncoefs, int nin, int elem_bytes) {
+    return elem_bytes == 16 ? blocks_of<double2>(g, range, ncoefs, nin)
+                            : blocks_of<double>(g, range, ncoefs, nin);
 }
 
 }  // namespace gb

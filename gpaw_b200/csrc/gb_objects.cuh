@@ -135,7 +135,7 @@ namespace gb {
 // Partial sums produced per grid by a residual sweep of `op`.
 inline int op_resid_blocks(const gb_operator* op, int nin, int es) {
     return op->tiled ? cfd_blocks(op->g, op->nn, es, nin, op->chunk) 
-           : op->general ? general_blocks(op->g, op->st.range, nin, es) : residual_blocks(op->g);
+           : op->general ? general_blocks(op->g, op->st.range, op->st.ncoefs, nin, es) : residual_blocks(op->g);
 }
 
 // One pass of the stencil with a fused epilogue; plane-marching kernel for

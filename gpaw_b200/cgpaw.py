@@ -21,11 +21,23 @@ from . import _lib
 from ._lib import GB_C128, GB_F64, check, f64, i64, phases_arg
 
 
+# The current stream's handle, and the device it is asked for, without the
+# Stream object that torch.cuda.current_stream() builds (1.3 of the 10 us of
+# a small apply).
+_raw_stream = getattr(torch._C, '_cuda_getCurrentRawStream', None)
+
+
 def _stream():
+    if _raw_stream is not None:
+        return C.c_void_p(_raw_stream(torch.cuda.current_device()))
     return C.c_void_p(torch.cuda.current_stream().cuda_stream)
 
 
 def _dtype_code(dtype):
+    if dtype is torch.float64:
+        return GB_F64
+    if dtype is torch.complex128:
+        return GB_C128
     if dtype in (float, np.float64, torch.float64, np.dtype('float64')):
         return GB_F64
     if dtype in (complex, np.complex128, torch.complex128,
@@ -35,6 +47,8 @@ def _dtype_code(dtype):
 
 
 def _check_tensor(a, name):
+    if isinstance(a, torch.Tensor) and a.is_cuda and a.is_contiguous():
+        return
     if not isinstance(a, torch.Tensor):
         raise TypeError(f'{name}: expected a torch CUDA tensor, got {type(a)}')
     if not a.is_cuda:
@@ -82,9 +96,11 @@ class Operator:
     def apply_gpu(self, in_ptr, out_ptr, shape, dtype, phases=None):
         """Operator_apply_gpu (c/gpu/operators.cpp:344-385)."""
         ph, ph_p = phases_arg(phases)
-        check(self._lib.gb_operator_apply(
-            self._h, C.c_void_p(in_ptr), C.c_void_p(out_ptr), _nin(shape),
-            _dtype_code(dtype), ph_p, _stream()))
+        rc = self._lib.gb_operator_apply(
+            self._h, in_ptr, out_ptr, _nin(shape), _dtype_code(dtype), ph_p,
+            _stream())
+        if rc:
+            check(rc)
 
     def relax_gpu(self, relax_method, f_ptr, s_ptr, nrelax, w=1.0):
         """Operator_relax_gpu (c/gpu/operators.cpp:200-221)."""
@@ -96,13 +112,14 @@ class Operator:
     def apply(self, input, output, phases=None):
         _check_tensor(input, 'input')
         _check_tensor(output, 'output')
-        if input.shape != output.shape or input.dtype != output.dtype:
+        shape, dtype = input.shape, input.dtype
+        if shape != output.shape or dtype != output.dtype:
             raise TypeError('input and output differ in shape or dtype')
-        if tuple(input.shape[-3:]) != self.size:
-            raise TypeError(f'grid shape {tuple(input.shape[-3:])} != '
+        if shape[-3:] != self.size:
+            raise TypeError(f'grid shape {tuple(shape[-3:])} != '
                             f'{self.size}')
-        self.apply_gpu(input.data_ptr(), output.data_ptr(),
-                       tuple(input.shape), input.dtype, phases)
+        self.apply_gpu(input.data_ptr(), output.data_ptr(), shape, dtype,
+                       phases)
 
     def apply_potential(self, input, output, v, phases=None):
         """output = L input + input * v (v: float64 grid shared by the
@@ -290,7 +307,7 @@ class Transformer:
             self._h, C.c_void_p(in_ptr), C.c_void_p(out_ptr), _nin(shape),
             _dtype_code(dtype), ph_p, _stream()))
 
-    def apply(self, input, output, phases=None):
+    def check_arrays(self, input, output):
         _check_tensor(input, 'input')
         _check_tensor(output, 'output')
         if tuple(input.shape[-3:]) != self.size_in or \
@@ -299,6 +316,9 @@ class Transformer:
         if input.shape[:-3] != output.shape[:-3] or \
                 input.dtype != output.dtype:
             raise TypeError('transformer: batch shape or dtype mismatch')
+
+    def apply(self, input, output, phases=None):
+        self.check_arrays(input, output)
         self.apply_gpu(input.data_ptr(), output.data_ptr(),
                        tuple(input.shape), input.dtype, phases)
 

@@ -57,6 +57,10 @@ SIGNATURES = {
                                      _i64p, _i64p, C.c_int, C.c_int,
                                      C.POINTER(_p)]),
     'gb_transformer_free': (None, [_p]),
+    'gb_density_work': (C.c_int64, [C.c_int64]),
+    'gb_density_interpolate': (C.c_int, [_p, _p, _p, C.c_int64,
+                                         C.POINTER(_p), C.c_double,
+                                         C.c_double, _p, _p]),
     'gb_transformer_apply': (C.c_int, [_p, _p, _p, C.c_int64, C.c_int, _dp,
                                        _p]),
     'gb_fd_precond': (C.c_int, [_p] * 7 + [_p] * 8 + [_p, _p, C.c_int64,

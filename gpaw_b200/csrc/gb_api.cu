@@ -472,6 +472,38 @@ extern "C" int gb_transformer_apply(gb_transformer* t, const void* in, void* out
     return transform_impl(t, in, out, nullptr, nin, dtype, P, 0, 0, 0.0, (cudaStream_t)stream);
 }
 
+namespace gb {
+int density_work_doubles(int nin);
+int launch_density(int k, const double* in, double* out, int nin, const XferGeom& G,
+                   const double* const w[3], double dv, double dvf, double* work,
+                   cudaStream_t st);
+}  // namespace gb
+
+extern "C" int64_t gb_density_work(int64_t nin) {
+    return nin > 0 && nin <= 65535 ? density_work_doubles((int)nin) : 0;
+}
+
+extern "C" int gb_density_interpolate(gb_transformer* t, const double* in, double* out,
+                                      int64_t nin, const double* const* weights, double dv,
+                                      double dv_fine, double* work, void* stream) {
+    if (!t || !in || !out || !weights || !weights[0] || !weights[1] || !weights[2] || !work)
+        return fail(GB_EINVAL, "density interpolate: NULL argument");
+    if (!t->interpolate || !t->real)
+        return fail(GB_EINVAL, "density interpolate: a real interpolator is needed");
+    if (nin <= 0) return 0;
+    if (nin > 65535) return fail(GB_EINVAL, "density interpolate: at most 65535 grids");
+    const char* ib = (const char*)in;
+    const char* ob = (const char*)out;
+    if (ib < ob + nin * t->ngout * 8 && ob < ib + nin * t->ngin * 8)
+        return fail(GB_EINVAL, "density interpolate: input and output overlap");
+    const int rc = launch_density(t->k, in, out, (int)nin, t->G, weights, dv, dv_fine, work,
+                                  (cudaStream_t)stream);
+    if (rc == -2) return fail(GB_ECUDA, "transformer: could not raise the shared-memory limit");
+    if (rc) return fail(GB_EINVAL, "transformer: unsupported order");
+    GB_LAUNCH_CHECK();
+    return 0;
+}
+
 // --------------------------------------------------------------- fd_precond
 extern "C" int gb_fd_precond(gb_transformer* rest0, gb_transformer* rest1, gb_transformer* intp1,
                              gb_transformer* intp2, gb_operator* kin0, gb_operator* kin1,

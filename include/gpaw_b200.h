@@ -243,6 +243,17 @@ GB_API void gb_transformer_free(gb_transformer* t);
 GB_API int gb_transformer_apply(gb_transformer* t, const void* in, void* out, int64_t nin,
                          int dtype, const double* phases, void* stream);
 
+/* Interpolation of nin float64 densities, each rescaled so that its fine
+ * integral equals the coarse one (FDPotentialCalculator._interpolate_density,
+ * gpaw/new/fd/pot_calc.py:72-80; left as it is where the fine integral is
+ * 1e-14 or less).  weights[c]: device array of the interpolator's column
+ * sums along axis c (the fine integral of a coarse value); dv, dv_fine: the
+ * volume elements; work: gb_density_work(nin) device doubles. */
+GB_API int64_t gb_density_work(int64_t nin);
+GB_API int gb_density_interpolate(gb_transformer* t, const double* in, double* out, int64_t nin,
+                                  const double* const* weights, double dv, double dv_fine,
+                                  double* work, void* stream);
+
 /* ---------------------------------------------------------------- fd_precond
  * Replaces cgpaw.fd_precond(rest0, rest1, intp1, intp2, kin0, kin1, kin2,
  * d0, q0, r1, d1, q1, r2, d2, q2, residuals, nresiduals, step, phases) —

@@ -1190,10 +1190,21 @@ int launch_density(int k, const double* in, double* out, int nin, const XferGeom
     return -1;
 }
 
+// order-2 transfers of real grids (gb_transfer2.cu)
+int launch_transfer2(bool interpolate, const double* in, double* out, double* out2, int nin,
+                     const XferGeom& G, cudaStream_t st);
+
 template <class T>
 int launch_transform(int k, bool interpolate, const void* in, void* out, void* out2, int nin,
                      const XferGeom& G, const Phases& P, cudaStream_t st) {
     const int K = k;
+    // (complex data stays with the kernels here: 16 x 40 x 48 x 36 coarse
+    // points took 66 against 43 us a restriction, 37 against 27 an
+    // interpolation, in registers)
+    if constexpr (sizeof(T) == 8)
+        if (k == 2 && launch_transfer2(interpolate, (const double*)in, (double*)out,
+                                       (double*)out2, nin, G, st) == 0)
+            return 0;
     if (interpolate) {
         switch (K) {
             case 2: return launch_interp_k<T, 2>(in, out, nin, G, P, st);

@@ -79,6 +79,12 @@ SIGNATURES = {
     'gb_woperator_relax': (C.c_int, [_p, C.c_int, _p, _p, C.c_int, C.c_double,
                                      _p]),
     'gb_woperator_get_diagonal_element': (C.c_int, [_p, _p, _p]),
+    'gb_wcoarse_new': (C.c_int, [C.c_int, C.POINTER(_p), C.POINTER(_p),
+                                 C.POINTER(_p), C.POINTER(C.c_int),
+                                 C.POINTER(C.c_int), _dp, C.POINTER(_p),
+                                 C.POINTER(_p), C.POINTER(_p)]),
+    'gb_wcoarse_free': (None, [_p]),
+    'gb_wcoarse_vcycle': (C.c_int, [_p, _p]),
     'gb_mixed_new': (C.c_int, [C.c_int, _p, C.POINTER(_p), C.POINTER(_p),
                                C.POINTER(_p), _dp, C.c_double, C.c_int,
                                C.POINTER(_p)]),

@@ -11,6 +11,7 @@
 #include <string>
 #include <vector>
 
+#include "gb_coarse.cuh"
 #include "gb_objects.cuh"
 #include "gb_tma.cuh"
 
@@ -611,254 +612,10 @@ __global__ void k_solve_init(SolveCtl* ctl, double eps, int maxiter) {
     ctl->err = 0.0;
 }
 
-// ------------------------------------------------ fused coarse-level V-cycle
-// The coarse levels of a multigrid hierarchy hold a few thousand points or
-// fewer, so each of their sweeps, residuals and transfers is one short
-// launch.  When every level from `lf` down is small, one CTA runs the whole
-// V-cycle below lf (iterate2 from level lf on, gpaw/poisson.py:500-537)
-// with all arrays in shared memory: weighted-Jacobi sweeps, the residual,
-// the K = 2 restriction and interpolation (three separable passes each, axis
-// 2, then 1, then 0, as bmgs_restrict / bmgs_interpolate order them,
-// c/bmgs/restrict.cpp:137-156, c/bmgs/interpolate.cpp:70-99).  Every value
-// is computed with the same operations in the same order as the per-level
-// kernels, so the V-cycle is bit-identical to them.
-namespace gb {
-constexpr int TAIL_MAX = 8;
-struct TailLevel {
-    int n[3];
-    int per[3];
-    int ng;
-    int phi, rho, tmp;        // offsets (doubles) of this level's arrays
-    double c0, cp[3], cm[3];  // 2nd-order stencil: direction k runs along axis 2 - k
-    int pre, post;
-    double w;
-    int rplo[3];              // restriction to the next level: input padding
-    double rw;                //   and mid-point weight
-    int iplo[3], iskip[3];    // interpolation from the next level: padding, skip
-    double iw;
-};
-struct TailPlan {
-    int nl;        // levels handled (lf .. L)
-    int scratch;   // offset of the transfer passes' intermediate arrays
-    TailLevel lv[TAIL_MAX];
-};
-
-// i / n for 0 <= i < 2^22 through a float reciprocal (inv = 1/n rounded):
-// the float quotient is within 1e-3 of i / n, so one correction step gives
-// the exact integer quotient
-__device__ __forceinline__ int tail_div(int i, int n, float inv) {
-    int q = __float2int_rz(__fmul_rn((float)i, inv));
-    const int r = i - q * n;
-    if (r < 0) q -= 1;
-    else if (r >= n) q += 1;
-    return q;
-}
-
-// index along one axis after the boundary condition; -1 reads zero
-__device__ __forceinline__ int tail_at(int j, int n, int per) {
-    if (j >= 0 && j < n) return j;
-    if (!per) return -1;
-    j = j < 0 ? j + n : j - n;
-    return (j >= 0 && j < n) ? j : -1;
-}
-
-// neighbour at +1 / -1 of point i (coordinate c, extent n, stride s)
-__device__ __forceinline__ double tail_up(const double* __restrict__ A, int i, int c, int n,
-                                          int per, int s) {
-    return (c + 1 < n) ? A[i + s] : (per ? A[i + s - n * s] : 0.0);
-}
-__device__ __forceinline__ double tail_dn(const double* __restrict__ A, int i, int c, int n,
-                                          int per, int s) {
-    return (c > 0) ? A[i - s] : (per ? A[i - s + n * s] : 0.0);
-}
-
-// x = 0 (+ v c0) + v(+1) c(+1) + v(-1) c(-1) per direction, axis 2, 1, 0
-template <bool CENTRE>
-__device__ __forceinline__ double tail_stencil(const double* __restrict__ A, const TailLevel& L,
-                                               int i, int i0, int i1, int i2) {
-    const int n1 = L.n[1], n2 = L.n[2];
-    double x = 0.0;
-    if (CENTRE) x = __dadd_rn(x, __dmul_rn(A[i], L.c0));
-    x = __dadd_rn(x, __dmul_rn(tail_up(A, i, i2, n2, L.per[2], 1), L.cp[0]));
-    x = __dadd_rn(x, __dmul_rn(tail_dn(A, i, i2, n2, L.per[2], 1), L.cm[0]));
-    x = __dadd_rn(x, __dmul_rn(tail_up(A, i, i1, n1, L.per[1], n2), L.cp[1]));
-    x = __dadd_rn(x, __dmul_rn(tail_dn(A, i, i1, n1, L.per[1], n2), L.cm[1]));
-    x = __dadd_rn(x, __dmul_rn(tail_up(A, i, i0, L.n[0], L.per[0], n1 * n2), L.cp[2]));
-    x = __dadd_rn(x, __dmul_rn(tail_dn(A, i, i0, L.n[0], L.per[0], n1 * n2), L.cm[2]));
-    return x;
-}
-
-// split a flat index of an (., b, c) array into its three coordinates
-__device__ __forceinline__ void tail_split(int i, int b, int c, float ibc, float ic, int& i0,
-                                           int& i1, int& i2) {
-    i0 = tail_div(i, b * c, ibc);
-    const int r = i - i0 * b * c;
-    i1 = tail_div(r, c, ic);
-    i2 = r - i1 * c;
-}
-
-// MODE 0: one weighted-Jacobi sweep A -> B (c/bmgs/relax.cpp:41-65);
-// MODE 1: the residual B = L A - rho
-template <int MODE>
-__device__ void tail_pass(const double* __restrict__ A, const double* __restrict__ R,
-                          double* __restrict__ B, const TailLevel& L) {
-    const int n1 = L.n[1], n2 = L.n[2];
-    const float i12 = __frcp_rn((float)(n1 * n2)), i2f = __frcp_rn((float)n2);
-    const double w1 = 1.0 - L.w;
-    for (int i = threadIdx.x; i < L.ng; i += blockDim.x) {
-        int i0, i1, i2;
-        tail_split(i, n1, n2, i12, i2f, i0, i1, i2);
-        if (MODE == 0) {
-            const double x = tail_stencil<false>(A, L, i, i0, i1, i2);
-            B[i] = __dadd_rn(__dmul_rn(w1, A[i]),
-                             __ddiv_rn(__dmul_rn(L.w, __dsub_rn(R[i], x)), L.c0));
-        } else {
-            B[i] = __dsub_rn(tail_stencil<true>(A, L, i, i0, i1, i2), R[i]);
-        }
-    }
-    __syncthreads();
-}
-
-// n weighted-Jacobi sweeps of the level's phi, held in buffer b (phi or
-// tmp); returns the buffer that holds the result
-__device__ __forceinline__ int tail_other(const TailLevel& L, int b) {
-    return b == L.phi ? L.tmp : L.phi;
-}
-__device__ __forceinline__ int tail_after(const TailLevel& L, int b, int n) {
-    return (n & 1) ? tail_other(L, b) : b;
-}
-__device__ int tail_relax(double* sm, const TailLevel& L, int b, int n) {
-    for (int it = 0; it < n; it++) {
-        tail_pass<0>(sm + b, sm + L.rho, sm + tail_other(L, b), L);
-        b = tail_other(L, b);
-    }
-    return b;
-}
-
-// mid-point restriction of one line value, K = 2: 0.5 (a + w (a+ + a-))
-__device__ __forceinline__ double tail_r1(const double* __restrict__ a, int j, int n, int per,
-                                          int s, double w) {
-    const int j0 = tail_at(j, n, per), jp = tail_at(j + 1, n, per), jm = tail_at(j - 1, n, per);
-    const double v = j0 < 0 ? 0.0 : a[j0 * s];
-    const double vp = jp < 0 ? 0.0 : a[jp * s];
-    const double vm = jm < 0 ? 0.0 : a[jm * s];
-    return __dmul_rn(0.5, __dadd_rn(v, __dmul_rn(w, __dadd_rn(vp, vm))));
-}
-
-// restriction of A (level F, extents n) into out (level C, extents m)
-__device__ void tail_restrict(const TailLevel& F, const TailLevel& C,
-                              const double* __restrict__ A, double* __restrict__ out,
-                              double* __restrict__ tA, double* __restrict__ tB) {
-    const int n0 = F.n[0], n1 = F.n[1], n2 = F.n[2];
-    const int m0 = C.n[0], m1 = C.n[1], m2 = C.n[2];
-    const float im2 = __frcp_rn((float)m2), im12 = __frcp_rn((float)(m1 * m2));
-    // axis 2: (n0, n1, m2)
-    for (int i = threadIdx.x; i < n0 * n1 * m2; i += blockDim.x) {
-        const int r = tail_div(i, m2, im2), c = i - r * m2;
-        tA[i] = tail_r1(A + r * n2, 2 * c + 1 - F.rplo[2], n2, F.per[2], 1, F.rw);
-    }
-    __syncthreads();
-    // axis 1: (n0, m1, m2)
-    for (int i = threadIdx.x; i < n0 * m1 * m2; i += blockDim.x) {
-        int i0, c1, c2;
-        tail_split(i, m1, m2, im12, im2, i0, c1, c2);
-        tB[i] = tail_r1(tA + i0 * n1 * m2 + c2, 2 * c1 + 1 - F.rplo[1], n1, F.per[1], m2, F.rw);
-    }
-    __syncthreads();
-    // axis 0: (m0, m1, m2)
-    for (int i = threadIdx.x; i < m0 * m1 * m2; i += blockDim.x) {
-        const int c0 = tail_div(i, m1 * m2, im12), r = i - c0 * m1 * m2;
-        out[i] = tail_r1(tB + r, 2 * c0 + 1 - F.rplo[0], n0, F.per[0], m1 * m2, F.rw);
-    }
-    __syncthreads();
-}
-
-// interpolated value at fine index f of one line a[j * s] of the coarse
-// level (length n, its boundary condition): the even outputs copy, the odd
-// ones are w (a(k) + a(k+1)) (c/bmgs/interpolate.cpp:10-46, K = 2)
-__device__ __forceinline__ double tail_i1(const double* __restrict__ a, int f, int skip, int plo,
-                                          int n, int per, int s, double w) {
-    const int u = f + skip;
-    const int k = u >> 1;
-    const int j = tail_at(k - plo, n, per);
-    const double v = j < 0 ? 0.0 : a[j * s];
-    if (!(u & 1)) return v;
-    const int j1 = tail_at(k + 1 - plo, n, per);
-    return __dmul_rn(w, __dadd_rn(v, j1 < 0 ? 0.0 : a[j1 * s]));
-}
-
-// phi (level F, extents n) -= interpolation of B (level C, extents m)
-__device__ void tail_interp_sub(const TailLevel& F, const TailLevel& C,
-                                const double* __restrict__ B, double* __restrict__ phi,
-                                double* __restrict__ tA, double* __restrict__ tB) {
-    const int n0 = F.n[0], n1 = F.n[1], n2 = F.n[2];
-    const int m0 = C.n[0], m1 = C.n[1], m2 = C.n[2];
-    const float in2 = __frcp_rn((float)n2), in12 = __frcp_rn((float)(n1 * n2));
-    // axis 2: (m0, m1, n2)
-    for (int i = threadIdx.x; i < m0 * m1 * n2; i += blockDim.x) {
-        const int r = tail_div(i, n2, in2), f = i - r * n2;
-        tA[i] = tail_i1(B + r * m2, f, F.iskip[2], F.iplo[2], m2, C.per[2], 1, F.iw);
-    }
-    __syncthreads();
-    // axis 1: (m0, n1, n2)
-    for (int i = threadIdx.x; i < m0 * n1 * n2; i += blockDim.x) {
-        int c0, f1, f2;
-        tail_split(i, n1, n2, in12, in2, c0, f1, f2);
-        tB[i] = tail_i1(tA + c0 * m1 * n2 + f2, f1, F.iskip[1], F.iplo[1], m1, C.per[1], n2,
-                        F.iw);
-    }
-    __syncthreads();
-    // axis 0: (n0, n1, n2), subtracted from phi
-    for (int i = threadIdx.x; i < n0 * n1 * n2; i += blockDim.x) {
-        const int f0 = tail_div(i, n1 * n2, in12), r = i - f0 * n1 * n2;
-        const double v = tail_i1(tB + r, f0, F.iskip[0], F.iplo[0], m0, C.per[0], n1 * n2, F.iw);
-        phi[i] = __dsub_rn(phi[i], v);
-    }
-    __syncthreads();
-}
-
-// The V-cycle from level lf down: rho_g is that level's right-hand side,
-// phi_g receives its correction (the level starts from zero).
-__global__ void __launch_bounds__(1024, 1)
-k_tail_vcycle(const double* __restrict__ rho_g, double* __restrict__ phi_g, TailPlan plan) {
-    extern __shared__ __align__(16) double tail_sm[];
-    double* sm = tail_sm;
-    const TailLevel& L0 = plan.lv[0];
-    for (int i = threadIdx.x; i < L0.ng; i += blockDim.x) {
-        sm[L0.rho + i] = rho_g[i];
-        sm[L0.phi + i] = 0.0;
-    }
-    __syncthreads();
-    double* tA = sm + plan.scratch;
-    const int last = plan.nl - 1;
-    for (int l = 0; l < last; l++) {
-        const TailLevel& L = plan.lv[l];
-        const TailLevel& C = plan.lv[l + 1];
-        const int cur = tail_relax(sm, L, L.phi, L.pre);
-        const int fre = tail_other(L, cur);
-        tail_pass<1>(sm + cur, sm + L.rho, sm + fre, L);
-        tail_restrict(L, C, sm + fre, sm + C.rho, tA, tA + L.n[0] * L.n[1] * C.n[2]);
-        for (int i = threadIdx.x; i < C.ng; i += blockDim.x) sm[C.phi + i] = 0.0;
-        __syncthreads();
-    }
-    const TailLevel& LL = plan.lv[last];
-    int fin = tail_relax(sm, LL, LL.phi, LL.post);
-    for (int l = last - 1; l >= 0; l--) {
-        const TailLevel& L = plan.lv[l];
-        const TailLevel& C = plan.lv[l + 1];
-        const int cur = tail_after(L, L.phi, L.pre);
-        tail_interp_sub(L, C, sm + fin, sm + cur, tA, tA + C.n[0] * C.n[1] * L.n[2]);
-        fin = tail_relax(sm, L, cur, L.post);
-    }
-    for (int i = threadIdx.x; i < L0.ng; i += blockDim.x) phi_g[i] = sm[fin + i];
-}
-}  // namespace gb
-
 struct gb_poisson {
     int L;  // coarsest level index
     int tail_lf = -1;           // first level of the fused coarse V-cycle (-1: none)
-    size_t tail_smem = 0;
-    gb::TailPlan tail;
+    gb::CoarsePlan tail;
     std::vector<gb_operator*> ops;
     std::vector<gb_transformer*> rst, itp;
     std::vector<int> pre, post;
@@ -896,113 +653,50 @@ struct gb_poisson {
     }
 };
 
-// Pick the first level of the fused coarse V-cycle: the coarsest run of
-// levels (below level 0) whose operators are 2nd-order axis-aligned
-// Laplacians, whose transfers are K = 2, that relax by weighted Jacobi,
-// whose first level holds at most TAIL_POINTS points and whose arrays fit
-// in shared memory.  GPAW_B200_POISSON_TAIL=0 keeps every level on the
-// per-level kernels (same results).
+// Pick the first level of the fused coarse V-cycle (gb_coarse.cu): the
+// coarsest run of levels (below level 0) whose operators are 2nd-order
+// axis-aligned Laplacians, whose transfers are K = 2, that relax by weighted
+// Jacobi and whose first level holds at most coarse_points() points (four a
+// thread; the 63^3 level of a 127^3 grid is faster over all SMs).
+// GPAW_B200_POISSON_TAIL=0 keeps every level on the per-level kernels (same
+// results).
 static void plan_tail(gb_poisson* p) {
-    constexpr long long TAIL_POINTS = 4096;
-    constexpr size_t TAIL_SMEM = 200 * 1024;
     p->tail_lf = -1;
+    memset(&p->tail, 0, sizeof p->tail);
     const char* env = getenv("GPAW_B200_POISSON_TAIL");
     if ((env && atoi(env) == 0) || p->method != 2 || p->L < 1) return;
-    auto level_ok = [&](int l) {
-        const gb_operator* op = p->ops[l];
-        if (!op->tiled || op->nn != 1 || !op->real) return false;
-        if (!(op->cs.axis[0] == 2 && op->cs.axis[1] == 1 && op->cs.axis[2] == 0)) return false;
-        if (l < p->L) {
-            const gb_transformer* r = p->rst[l];
-            const gb_transformer* i = p->itp[l];
-            if (r->k != 2 || i->k != 2) return false;
-            for (int c = 0; c < 3; c++) {
-                if (r->G.g.n[c] != op->g.n[c] || r->G.g.periodic[c] != op->g.periodic[c] ||
-                    r->G.nout[c] != p->ops[l + 1]->g.n[c] ||
-                    i->G.g.n[c] != p->ops[l + 1]->g.n[c] ||
-                    i->G.g.periodic[c] != p->ops[l + 1]->g.periodic[c] ||
-                    i->G.nout[c] != op->g.n[c])
-                    return false;
-            }
-        }
-        return true;
-    };
-    auto smem_from = [&](int lf) {
-        size_t d = 0, scratch = 0;
-        for (int l = lf; l <= p->L; l++) {
-            d += 3 * (size_t)p->ops[l]->ng();
-            if (l < p->L) {
-                const int* n = p->ops[l]->g.n;
-                const int* m = p->ops[l + 1]->g.n;
-                const size_t r = (size_t)n[0] * n[1] * m[2] + (size_t)n[0] * m[1] * m[2];
-                const size_t i = (size_t)m[0] * m[1] * n[2] + (size_t)m[0] * n[1] * n[2];
-                scratch = std::max(scratch, std::max(r, i));
-            }
-        }
-        return (d + scratch) * sizeof(double);
-    };
+    std::vector<gb::CoarseLevel> lv(p->L + 1);
     int lf = -1;
     for (int l = p->L; l >= 1; l--) {
-        if (!level_ok(l) || p->ops[l]->ng() > TAIL_POINTS || smem_from(l) > TAIL_SMEM ||
-            p->L - l + 1 > gb::TAIL_MAX)
-            break;
-        lf = l;
-    }
-    if (lf < 0) return;
-    gb::TailPlan& T = p->tail;
-    memset(&T, 0, sizeof T);
-    T.nl = p->L - lf + 1;
-    int off = 0;
-    for (int k = 0; k < T.nl; k++) {
-        const int l = lf + k;
         const gb_operator* op = p->ops[l];
-        gb::TailLevel& V = T.lv[k];
+        if (!op->tiled || op->nn != 1 || !op->real || op->ng() > gb::coarse_points(false) ||
+            !(op->cs.axis[0] == 2 && op->cs.axis[1] == 1 && op->cs.axis[2] == 0) ||
+            p->L - l + 1 > gb::COARSE_LEVELS)
+            break;
+        gb::CoarseLevel& V = lv[l];
+        memset(&V, 0, sizeof V);
         V.ng = (int)op->ng();
         for (int c = 0; c < 3; c++) {
             V.n[c] = op->g.n[c];
             V.per[c] = op->g.periodic[c];
+            V.cp[c] = op->cs.cp[c][0];
+            V.cm[c] = op->cs.cm[c][0];
         }
-        V.phi = off;
-        V.rho = off + V.ng;
-        V.tmp = off + 2 * V.ng;
-        off += 3 * V.ng;
         V.c0 = op->cs.c0;
-        for (int d = 0; d < 3; d++) {
-            V.cp[d] = op->cs.cp[d][0];
-            V.cm[d] = op->cs.cm[d][0];
-        }
+        V.rc0 = 1.0 / op->cs.c0;
         V.pre = p->pre[l];
         V.post = p->post[l];
-        V.w = p->w[l];
-        if (l < p->L) {
-            const gb_transformer* r = p->rst[l];
-            const gb_transformer* i = p->itp[l];
-            for (int c = 0; c < 3; c++) {
-                V.rplo[c] = r->G.plo[c];
-                V.iplo[c] = i->G.plo[c];
-                V.iskip[c] = i->G.skip0[c];
-            }
-            V.rw = r->G.w[0];
-            V.iw = i->G.w[0];
-        }
+        V.wj = p->w[l];
+        if (l < p->L &&
+            !gb::coarse_transfers(V, p->rst[l]->k, p->rst[l]->G, p->itp[l]->k, p->itp[l]->G,
+                                  p->ops[l + 1]->g.n))
+            break;
+        lf = l;
     }
-    T.scratch = off;
-    p->tail_smem = smem_from(lf);
+    if (lf < 0) return;
+    p->tail.nl = p->L - lf + 1;
+    for (int l = lf; l <= p->L; l++) p->tail.lv[l - lf] = lv[l];
     p->tail_lf = lf;
-}
-
-static int launch_tail(gb_poisson* p, cudaStream_t st) {
-    static bool attr_done = false;
-    if (!attr_done) {
-        GB_CUDA_TRY(cudaFuncSetAttribute(gb::k_tail_vcycle,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         227 * 1024));
-        attr_done = true;
-    }
-    const int lf = p->tail_lf;
-    gb::k_tail_vcycle<<<1, 1024, p->tail_smem, st>>>(p->rho[lf], p->phi[lf], p->tail);
-    GB_LAUNCH_CHECK();
-    return 0;
 }
 
 extern "C" int gb_poisson_new(int nlevels, gb_operator* const* operators,
@@ -1076,6 +770,12 @@ extern "C" int gb_poisson_new(int nlevels, gb_operator* const* operators,
         delete p;
         return fail(GB_ECUDA, "Poisson: allocation: %s", cudaGetErrorString(e));
     }
+    for (int k = 0; k < p->tail.nl; k++) {
+        gb::CoarseLevel& V = p->tail.lv[k];
+        V.phi = p->phi[p->tail_lf + k];
+        V.rho = p->rho[p->tail_lf + k];
+        V.tmp = p->res[p->tail_lf + k];
+    }
     *out = p;
     return 0;
 }
@@ -1088,7 +788,7 @@ extern "C" int gb_poisson_fused_levels(const gb_poisson* p) {
 
 // iterate2 (gpaw/poisson.py:500-537), recursive over levels.
 static int vcycle(gb_poisson* p, int l, cudaStream_t st) {
-    if (l == p->tail_lf) return launch_tail(p, st);   // starts from phi_l = 0 itself
+    if (l == p->tail_lf) return launch_coarse(p->tail, false, st);   // starts from phi_l = 0
     gb_operator* op = p->ops[l];
     Phases P;
     memset(&P, 0, sizeof P);

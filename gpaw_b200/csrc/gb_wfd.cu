@@ -16,6 +16,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "gb_coarse.cuh"
 #include "gb_objects.cuh"
 
 using namespace gb;
@@ -738,4 +739,92 @@ extern "C" int gb_woperator_get_diagonal_element(gb_woperator* op, double* out, 
     memcpy(&d, &bits, sizeof d);
     *out = d;
     return 0;
+}
+
+// ------------------------------------------------------ fused coarse levels
+// The coarse levels of the dielectric solver's V-cycle in one launch
+// (gb_coarse.cu): operators [Laplacian, three derivatives] of second order,
+// each level's arrays given by the caller (weights through the operators).
+struct gb_wcoarse {
+    CoarsePlan plan;
+    double* tmp = nullptr;
+    ~gb_wcoarse() { dfree(tmp); }
+};
+
+static bool wcoarse_level(const gb_woperator* op, CoarseLevel& L) {
+    WGroups G;
+    if (!op->real || op->s.nw != 4 || op->s.range != 1 || !op->s.cfd ||
+        !wfd_groups(op->s, 1, G) || G.ng[0] != 3)
+        return false;
+    L.ng = (int)op->ng();
+    for (int c = 0; c < 3; c++) {
+        L.n[c] = op->g.n[c];
+        L.per[c] = op->g.periodic[c];
+        if (G.axis[0][c] != 2 - c || G.ng[c + 1] != 1) return false;
+        L.cp[c] = G.cp[0][c][0];
+        L.cm[c] = G.cm[0][c][0];
+        L.gaxis[c] = G.axis[c + 1][0];
+        L.gc0[c] = G.c0[c + 1];
+        L.gp[c] = G.cp[c + 1][0][0];
+        L.gm[c] = G.cm[c + 1][0][0];
+    }
+    L.c0 = G.c0[0];
+    for (int i = 0; i < 4; i++) L.w[i] = op->s.w[i];
+    return true;
+}
+
+extern "C" int gb_wcoarse_new(int nlevels, gb_woperator* const* ops,
+                              gb_transformer* const* restrictors,
+                              gb_transformer* const* interpolators, const int* pre,
+                              const int* post, const double* weights, double* const* phi,
+                              double* const* rho, gb_wcoarse** out) {
+    if (!out || !ops || !pre || !post || !weights || !phi || !rho || nlevels < 1 ||
+        (nlevels > 1 && (!restrictors || !interpolators)))
+        return fail(GB_EINVAL, "wcoarse: bad arguments");
+    *out = nullptr;
+    if (nlevels > COARSE_LEVELS) return 0;
+    gb_wcoarse* w = new gb_wcoarse();
+    memset(&w->plan, 0, sizeof w->plan);
+    w->plan.nl = nlevels;
+    size_t total = 0;
+    bool ok = true;
+    for (int l = 0; l < nlevels && ok; l++) {
+        CoarseLevel& L = w->plan.lv[l];
+        ok = ops[l] && phi[l] && rho[l] && wcoarse_level(ops[l], L);
+        if (!ok) break;
+        L.phi = phi[l];
+        L.rho = rho[l];
+        L.pre = pre[l];
+        L.post = post[l];
+        L.wj = weights[l];
+        if (l + 1 < nlevels) {
+            const gb_transformer *r = restrictors[l], *i = interpolators[l];
+            ok = ops[l + 1] && r && i && r->real && i->real && !r->interpolate &&
+                 i->interpolate &&
+                 coarse_transfers(L, r->k, r->G, i->k, i->G, ops[l + 1]->g.n);
+        }
+        total += (L.ng + 31) / 32 * 32;
+    }
+    if (!ok || w->plan.lv[0].ng > coarse_points(true)) {
+        delete w;          // the caller keeps its per-level launches
+        return 0;
+    }
+    if (int rc = dmalloc((void**)&w->tmp, total * sizeof(double))) {
+        delete w;
+        return rc;
+    }
+    double* t = w->tmp;
+    for (int l = 0; l < nlevels; l++) {
+        w->plan.lv[l].tmp = t;
+        t += (w->plan.lv[l].ng + 31) / 32 * 32;
+    }
+    *out = w;
+    return 0;
+}
+
+extern "C" void gb_wcoarse_free(gb_wcoarse* w) { delete w; }
+
+extern "C" int gb_wcoarse_vcycle(gb_wcoarse* w, void* stream) {
+    if (!w) return fail(GB_EINVAL, "wcoarse: NULL object");
+    return launch_coarse(w->plan, true, (cudaStream_t)stream);
 }

@@ -19,11 +19,15 @@ Charged periodic systems raise NotImplementedError, as in the reference.
 """
 from __future__ import annotations
 
+import ctypes as C
+
 import numpy as np
 import torch
 from scipy.special import erf
 
+from . import _lib
 from ._lib import PoissonConvergenceError
+from .cgpaw import _stream
 from .fd_operators import Gradient, Laplace
 from .gauss import SQRT_PI, coordinates
 from .poisson import FDPoissonSolver, _solve_monopole
@@ -87,6 +91,7 @@ class WeightedFDPoissonSolver(FDPoissonSolver):
         level = self.levels
         self.presmooths[level] = 8
         self.postsmooths[level] = 8
+        self._coarse = _CoarseLevels.build(self)
         self._initialized = True
 
     def restrict_op_weights(self):
@@ -190,6 +195,9 @@ class WeightedFDPoissonSolver(FDPoissonSolver):
 
     def _cycle_no_read(self, level):
         """iterate2's V-cycle below `level` without the final host read."""
+        if self._coarse is not None and level == self._coarse.first:
+            self._coarse.vcycle()         # from phi = 0, in one launch
+            return
         residual = self.residuals[level]
         op = self.operators[level]
         if level < self.levels:
@@ -198,7 +206,8 @@ class WeightedFDPoissonSolver(FDPoissonSolver):
             op.apply(self.phis[level], residual)
             residual -= self.rhos[level]
             self.restrictors[level].apply(residual, self.rhos[level + 1])
-            self.phis[level + 1].zero_()
+            if self._coarse is None or level + 1 != self._coarse.first:
+                self.phis[level + 1].zero_()
             self._cycle_no_read(level + 1)
             self.interpolators[level].apply(self.phis[level + 1], residual)
             self.phis[level] -= residual
@@ -268,3 +277,59 @@ class WeightedFDPoissonSolver(FDPoissonSolver):
             residual -= self.rhos[level]
             r = residual.reshape(-1)
             return float(torch.dot(r, r)) * self.gd.dv
+
+
+class _CoarseLevels:
+    """The coarse levels of a solver's captured V-cycle as one launch
+    (gb_wcoarse_*): the longest run of levels below level 0, down to the
+    coarsest, that the library takes (second-order orthorhombic operators,
+    weighted Jacobi, at most 32768 points)."""
+
+    MAX_LEVELS = 8
+
+    @classmethod
+    def build(cls, solver):
+        if solver.relax_method != 2 or not solver.phis[-1:] or \
+                solver.levels < 1 or not solver.rhos[-1].is_cuda:
+            return None
+        for first in range(1, solver.levels + 1):
+            if int(np.prod(solver.operators[first].gd.n_c)) <= 32768 and \
+                    solver.levels - first + 1 <= cls.MAX_LEVELS:
+                obj = cls(solver, first)
+                return obj if obj._h.value else None
+        return None
+
+    def __init__(self, solver, first):
+        levels = range(first, solver.levels + 1)
+        n = len(levels)
+        ops = [solver.operators[l] for l in levels]
+        rst = [solver.restrictors[l] for l in levels[:-1]]
+        itp = [solver.interpolators[l] for l in levels[:-1]]
+        phi = [solver.phis[l] for l in levels]
+        rho = [solver.rhos[l] for l in levels]
+        self._keep = (ops, rst, itp, phi, rho)
+        self.first = first
+        lib = self._lib = _lib.load()
+
+        def pointers(handles):
+            return (C.c_void_p * max(1, len(handles)))(*handles)
+
+        self._h = C.c_void_p()
+        _lib.check(lib.gb_wcoarse_new(
+            n, pointers([o.operator._h for o in ops]),
+            pointers([t.transformer._h for t in rst]),
+            pointers([t.transformer._h for t in itp]),
+            (C.c_int * n)(*[solver.presmooths[l] for l in levels]),
+            (C.c_int * n)(*[solver.postsmooths[l] for l in levels]),
+            (C.c_double * n)(*[solver.weights[l] for l in levels]),
+            pointers([t.data_ptr() for t in phi]),
+            pointers([t.data_ptr() for t in rho]), C.byref(self._h)))
+
+    def __del__(self):
+        h = getattr(self, '_h', None)
+        if h is not None and h.value:
+            self._lib.gb_wcoarse_free(h)
+            self._h = None
+
+    def vcycle(self):
+        _lib.check(self._lib.gb_wcoarse_vcycle(self._h, _stream()))

@@ -224,6 +224,25 @@ GB_API int gb_woperator_relax(gb_woperator* op, int method, double* f, const dou
  * *out (host).  Synchronises the stream. */
 GB_API int gb_woperator_get_diagonal_element(gb_woperator* op, double* out, void* stream);
 
+/* The coarse levels of the dielectric solver's V-cycle in one launch:
+ * iterate2 (gpaw/poisson.py:500-537) from operators[0] on, starting from
+ * phi = 0, on the caller's arrays: reads rho[0], leaves the correction in
+ * phi[0], uses the other levels' phi and rho as work arrays.  Levels as
+ * WeightedFDPoissonSolver builds them (a second-order Laplacian and the three
+ * derivatives; order-2 transfers; weighted Jacobi with pre/post sweeps and
+ * the given relaxation weights); bit-identical to the per-level calls.
+ * gb_wcoarse_new returns 0 with *out = NULL for levels it does not take (the
+ * first may have 32768 points).  Operators, transformers and arrays must
+ * outlive the object.  No reference counterpart. */
+typedef struct gb_wcoarse gb_wcoarse;
+GB_API int gb_wcoarse_new(int nlevels, gb_woperator* const* operators,
+                          gb_transformer* const* restrictors,
+                          gb_transformer* const* interpolators, const int* pre, const int* post,
+                          const double* weights, double* const* phi, double* const* rho,
+                          gb_wcoarse** out);
+GB_API void gb_wcoarse_free(gb_wcoarse* w);
+GB_API int gb_wcoarse_vcycle(gb_wcoarse* w, void* stream);
+
 /* --------------------------------------------------------------- Transformer
  * Replaces cgpaw.Transformer(size_in, size_out, k, pads, npads, skip,
  * neighbors, real, comm, interpolate, use_gpu) — NewTransformerObject,

@@ -66,18 +66,26 @@ class FDDensityTransfers:
         self.interpolation_stencil_range = n
         self._interpolate = Transformer(gd, finegd, n, dtype)
         self._restrict = Transformer(finegd, gd, n, dtype)
-        self._weights = None      # on the device (built on first use)
+        # the column sums go to the device now, so that a first call may be
+        # under a stream capture
+        self._weights = None
+        if getattr(self._interpolate, 'dtype', None) is float and \
+                not bool(gd.pbc_c.all()) and torch.cuda.is_available():
+            self._upload_column_sums()
+
+    def _upload_column_sums(self):
+        t = self._interpolate
+        w = [interpolation_column_sums(
+            t.ngpin[c], t.ngpout[c], bool(self.grid.pbc_c[c]),
+            int(t.pad_cd[c, 0]), int(t.skip_cd[c, 0]), t.nn)
+            for c in range(3)]
+        self._weights = torch.from_numpy(np.concatenate(w)).to(
+            self.grid.device)
 
     def _column_sums(self):
         """Device addresses of the three axes' column sums."""
         if self._weights is None:
-            t = self._interpolate
-            w = [interpolation_column_sums(
-                t.ngpin[c], t.ngpout[c], bool(self.grid.pbc_c[c]),
-                int(t.pad_cd[c, 0]), int(t.skip_cd[c, 0]), t.nn)
-                for c in range(3)]
-            self._weights = torch.from_numpy(np.concatenate(w)).to(
-                self.grid.device)
+            self._upload_column_sums()
         p = self._weights.data_ptr()
         n = self._interpolate.ngpin
         return (C.c_void_p * 3)(p, p + 8 * n[0], p + 8 * (n[0] + n[1]))

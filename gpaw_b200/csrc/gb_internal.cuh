@@ -116,7 +116,7 @@ template <class T>
 int launch_general(int mode, const void* in, void* out, int nin, const GridBC& g,
                    const Phases& P, const Stencil& st, const Epi& ep, cudaStream_t stream);
 int general_blocks(const GridBC& g, int range, int ncoefs, int nin, int elem_bytes);
-int cfd_chunk(const GridBC& g, int nn, int nin, int ty);
+int cfd_chunk(const GridBC& g, int nn, int nin, int ty, int per_sm = 4);
 // read and clear the device fault flag of a kernel file (bounded waits)
 int take_fault_transform(int* code);
 int take_fault_cfd(int* code);

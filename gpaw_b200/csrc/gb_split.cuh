@@ -24,4 +24,12 @@ inline int split_planes(int n, int step, int extra, long long tiles, long long s
     return chunk;
 }
 
+// The chunk halved until `tiles` column tiles make `target` CTAs, at least
+// `least` planes.
+inline int halve_planes(int n, int least, long long tiles, long long target) {
+    int c = n;
+    while (c > least && tiles * ((n + c - 1) / c) < target) c = (c + 1) / 2;
+    return c;
+}
+
 }  // namespace gb

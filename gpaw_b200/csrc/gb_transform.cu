@@ -1034,11 +1034,15 @@ static int launch_restrict_k(const void* in, void* out, void* out2, int nin, con
         attr = true;
     }
     const int t1 = (G.nout[1] + TJ - 1) / TJ, t2 = (G.nout[2] + TK - 1) / TK;
-    // (three CTAs an SM, fewer where their shared memory is large)
+    // (three CTAs an SM, fewer where their shared memory is large; complex
+    // grids keep many short chunks: 16 x 80 x 96 x 72, K = 2, 43 us against
+    // 46)
     const int per_sm = std::max(1, std::min(3, (int)(227 * 1024 / (smem + 1024))));
+    const long long tiles = (long long)t1 * t2 * nin;
     const int chunk0 = G.chunk > 0 ? std::min(G.chunk, G.nout[0])
-                                   : split_planes(G.nout[0], 2, 2 * K - 3 + 8,
-                                                  (long long)t1 * t2 * nin, 148 * per_sm);
+                       : sizeof(T) == 16 ? halve_planes(G.nout[0], 4, tiles, 148 * 4)
+                                         : split_planes(G.nout[0], 2, 2 * K - 3 + 8, tiles,
+                                                        148 * per_sm);
     const int nchunks = (G.nout[0] + chunk0 - 1) / chunk0;
     for (int b0 = 0; b0 < nin; b0 += 65535) {
         const int nb = min(65535, nin - b0);
@@ -1080,9 +1084,11 @@ static int launch_interp_v(const void* in, void* out, int nin, const XferGeom& G
     const int t1 = (G.nout[1] + TJ - 1) / TJ, t2 = (G.nout[2] + TK - 1) / TK;
     const int n0p = G.s[0] - (K - 1) + G.skip1[0];
     const int per_sm = std::max(1, std::min(4, (int)(227 * 1024 / (smem + 1024))));
+    // (complex: as for the restriction, 28 us against 30)
+    const long long tiles = (long long)t1 * t2 * nin;
     const int chunk0 = G.chunk > 0 ? std::min(G.chunk, n0p)
-                                   : split_planes(n0p, 1, K - 1 + 8, (long long)t1 * t2 * nin,
-                                                  148 * per_sm);
+                       : sizeof(T) == 16 ? halve_planes(n0p, 4, tiles, 148 * 8)
+                                         : split_planes(n0p, 1, K - 1 + 8, tiles, 148 * per_sm);
     const int nchunks = (n0p + chunk0 - 1) / chunk0;
     for (int b0 = 0; b0 < nin; b0 += 65535) {
         const int nb = min(65535, nin - b0);

@@ -37,7 +37,8 @@ namespace gb {
 // per_sm CTAs an SM at once (GPAW_B200_CTA_TARGET=n: n CTAs in all); a CTA
 // reads 2 nn planes beyond its own.  Against halving the chunk until the
 // launch had 296 CTAs: 32 x 111 x 119 x 95 real H psi 334 -> 294 us (two
-// chunks make 4.9 full waves instead of 2.4 of long ones).
+// chunks make 4.9 full waves instead of 2.4 of long ones).  The complex kernels
+// (per_sm 0) keep that older rule: 16 x 40 x 48 x 36, nn = 1, 14 us against 18.
 int cfd_chunk(const GridBC& g, int nn, int nin, int ty, int per_sm) {
     static int target = [] {
         const char* v = getenv("GPAW_B200_CTA_TARGET");
@@ -45,8 +46,9 @@ int cfd_chunk(const GridBC& g, int nn, int nin, int ty, int per_sm) {
     }();
     const int tiles_x = (g.n[2] + 31) / 32;
     const int tiles_y = (g.n[1] + ty - 1) / ty;
-    return split_planes(g.n[0], 1, 2 * nn, (long long)tiles_x * tiles_y * nin,
-                        target > 0 ? target : 148 * per_sm);
+    const long long tiles = (long long)tiles_x * tiles_y * nin;
+    if (per_sm == 0) return halve_planes(g.n[0], 2 * nn, tiles, target > 0 ? target : 148 * 2);
+    return split_planes(g.n[0], 1, 2 * nn, tiles, target > 0 ? target : 148 * per_sm);
 }
 
 // GPAW_B200_FMA=1 selects the fused-multiply-add form of the complex
@@ -647,7 +649,7 @@ static int launch_cfd_t(const void* in, void* out, int nin, const GridBC& g, con
     }
     const int tiles_x = (g.n[2] + TX - 1) / TX;
     const int tiles_y = (g.n[1] + TY - 1) / TY;
-    const int chunk0 = ep.chunk > 0 ? min(ep.chunk, g.n[0]) : cfd_chunk(g, NN, nin, TY, sizeof(T) == 16 ? MINB : 4);
+    const int chunk0 = ep.chunk > 0 ? min(ep.chunk, g.n[0]) : cfd_chunk(g, NN, nin, TY, sizeof(T) == 16 ? 0 : 4);
     const int nch = (g.n[0] + chunk0 - 1) / chunk0;
     if (nblk) *nblk = tiles_x * tiles_y * nch;
     const long long ng = (long long)g.n[0] * g.n[1] * g.n[2];
@@ -809,7 +811,7 @@ int cfd_blocks(const GridBC& g, int nn, int elem_bytes, int nin, int chunk) {
     const int TX = 32, TY = elem_bytes == 4 ? 16 : 8;
     const int tiles_x = (g.n[2] + TX - 1) / TX;
     const int tiles_y = (g.n[1] + TY - 1) / TY;
-    const int chunk0 = chunk > 0 ? std::min(chunk, g.n[0]) : cfd_chunk(g, nn, nin, TY, elem_bytes == 16 ? 2 : 4);   // EPI_RESID
+    const int chunk0 = chunk > 0 ? std::min(chunk, g.n[0]) : cfd_chunk(g, nn, nin, TY, elem_bytes == 16 ? 0 : 4);
     return tiles_x * tiles_y * ((g.n[0] + chunk0 - 1) / chunk0);
 }
 

@@ -509,7 +509,7 @@ static int launch_wfd_tiled_k(const void* in, void* out, int nin, const GridBC& 
     }
     const int tiles_x = (g.n[2] + WX - 1) / WX;
     const int tiles_y = (g.n[1] + WY - 1) / WY;
-    const int chunk0 = cfd_chunk(g, R, nin, WY);
+    const int chunk0 = cfd_chunk(g, R, nin, WY, sizeof(T) == 16 ? 0 : 4);
     const int nch = (g.n[0] + chunk0 - 1) / chunk0;
     const long long ng = (long long)g.n[0] * g.n[1] * g.n[2];
     for (int b0 = 0; b0 < nin; b0 += 65535) {

@@ -22,12 +22,11 @@
 // instead.
 #include "gb_direct.cuh"
 #include "gb_objects.cuh"
+#include "gb_stage.cuh"
 
 namespace gb {
 namespace {
 
-constexpr int PT_ROWS = 16;   // rows of a tile, 16 threads each
-constexpr int PT_HX = 4;      // halo columns staged on each side
 constexpr int PT_RING = 8;    // planes in the ring
 
 template <class T>
@@ -132,24 +131,15 @@ pass_body(const T* __restrict__ u, T* __restrict__ out, const T* __restrict__ au
     }
 
     // staging map: in-plane offset of each element this thread copies, or
-    // -1 for a zero (outside a zero boundary); the boundary is fixed per CTA
+    // -1 for a zero; the boundary is fixed per CTA
     int goff[NE];
 #pragma unroll
     for (int i = 0; i < NE; i++) {
         const int e = tid + 256 * i;
         goff[i] = -1;
         if (e < E) {
-            int r = y0 - NN + e / C, col = x0 - PT_HX + e % C;
-            bool ok = true;
-            if (r < 0 || r >= n1) {
-                if (g.periodic[1]) r += r < 0 ? n1 : -n1;
-                else ok = false;
-            }
-            if (col < 0 || col >= n2) {
-                if (g.periodic[2]) col += col < 0 ? n2 : -n2;
-                else ok = false;
-            }
-            if (ok) goff[i] = r * n2 + col;
+            goff[i] = staged_offset(y0 - NN + e / C, x0 - PT_HX + e % C, n1, n2, g.periodic[1],
+                                    g.periodic[2]);
         }
     }
     const unsigned ring_addr = (unsigned)__cvta_generic_to_shared(ring);

@@ -40,6 +40,7 @@ SIGNATURES = {
     'gb_operator_residual': (C.c_int, [_p, _p, _p, _p, C.c_int64, C.c_int,
                                        _dp, C.c_double, _p, _p]),
     'gb_operator_get_diagonal_element': (C.c_double, [_p]),
+    'gb_operator_path': (C.c_int, [_p]),
     'gb_trace_begin': (C.c_int, [C.c_int]),
     'gb_device_fault': (C.c_int, [C.POINTER(C.c_int)]),
     'gb_pool_set': (C.c_int, [C.c_int, C.c_size_t]),

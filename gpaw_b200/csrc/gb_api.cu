@@ -205,7 +205,10 @@ extern "C" int gb_operator_new(const double* coefs, const int64_t* offsets, int 
     }
     const char* path = getenv("GPAW_B200_FD_PATH");
     const bool force_generic = path && strcmp(path, "generic") == 0;
-    op->tiled = (!force_generic && to_cfd_stencil(op->st, op->cs, op->nn)) ? 1 : 0;
+    // (the plane-marching kernels sum axis 2, then 1, then 0: the order of
+    // every Laplacian; axis-aligned stencils in another order are general)
+    op->tiled = !force_generic && to_cfd_stencil(op->st, op->cs, op->nn) &&
+                op->cs.axis[0] == 2 && op->cs.axis[1] == 1 && op->cs.axis[2] == 0;
     bool axis_aligned = true;
     for (int p = 0; p < ncoefs; p++) {
         const int* o = op->st.off[p];
@@ -220,6 +223,10 @@ extern "C" void gb_operator_free(gb_operator* op) { delete op; }
 
 extern "C" double gb_operator_get_diagonal_element(const gb_operator* op) {
     return op ? op->diag : 0.0;
+}
+
+extern "C" int gb_operator_path(const gb_operator* op) {
+    return !op ? 0 : op->tiled ? 2 : op->general ? 1 : 0;
 }
 
 extern "C" int gb_operator_reserve(gb_operator* op, int64_t nin, int dtype) {

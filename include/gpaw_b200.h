@@ -177,6 +177,11 @@ GB_API int gb_operator_residual(gb_operator* op, const void* phi, const void* rh
 /* Replaces Operator.get_diagonal_element(), c/operators.cpp:319-332. */
 GB_API double gb_operator_get_diagonal_element(const gb_operator* op);
 
+/* The kernels that the operator runs on: 2 the plane-marching ones for
+ * Laplacian-like stencils, 1 the tiled ones for general stencils, 0 one thread
+ * a point.  The results are the same.  No reference counterpart. */
+GB_API int gb_operator_path(const gb_operator* op);
+
 /* Preallocate the operator's scratch for batches up to nin grids (so that
  * later calls allocate nothing, e.g. inside CUDA-graph capture). */
 GB_API int gb_operator_reserve(gb_operator* op, int64_t nin, int dtype);

@@ -75,3 +75,36 @@ def test_general_laplacian(cell, nn, cuda):
     out = to_dev(np.zeros_like(a))
     Laplace(gdp, -0.5, nn, complex).apply(to_dev(a), out, ph)
     assert np.array_equal(to_np(out), ref)
+
+
+@pytest.mark.parametrize('dtype', [float, complex])
+@pytest.mark.parametrize('nn', [1, 3])
+def test_axis_aligned_in_another_order(nn, dtype, cuda):
+    """Centre, then the axes in the order 0, 1, 2: laid out as a Laplacian is,
+    but not summed in its order.  The residual's norm has one partial sum for
+    each block of the kernel that runs (few or many planes, one grid or
+    more).  Tolerance: the sums' order, n eps."""
+    import torch
+    rng = np.random.default_rng(nn)
+    offsets = [(0, 0, 0)]
+    for axis in range(3):
+        for sign in (1, -1):
+            for d in range(1, nn + 1):
+                o = [0, 0, 0]
+                o[axis] = sign * d
+                offsets.append(tuple(o))
+    coefs = rng.standard_normal(len(offsets))
+    for N, nin in (((64, 64, 64), 1), ((10, 33, 70), 5), ((90, 12, 8), 2)):
+        gdp, op, gdo, oo = _pair(N, np.eye(3), (1, 0, 1), coefs, offsets,
+                                 dtype)
+        a = _data(rng, (nin,) + tuple(gdo.n_c), dtype)
+        rho = _data(rng, a.shape, dtype)
+        ref = np.zeros_like(a)
+        ph = gdo.phase_factor_cd((0.2, 0, 0.1)) if dtype is complex else None
+        oo.apply(a, ref, ph)
+        x, res = to_dev(a), to_dev(np.zeros_like(a))
+        norm = torch.zeros(nin, dtype=torch.float64, device='cuda')
+        op.operator.residual(x, to_dev(rho), res, ph, 0.5, norm)
+        assert np.array_equal(to_np(res), ref - rho)
+        want = 0.5 * (np.abs(ref - rho)**2).reshape(nin, -1).sum(1)
+        assert np.abs(to_np(norm) / want - 1).max() < 1e-13 * a[0].size**0.5

@@ -214,7 +214,7 @@ extern "C" int gb_operator_new(const double* coefs, const int64_t* offsets, int 
         const int* o = op->st.off[p];
         axis_aligned = axis_aligned && (o[0] != 0) + (o[1] != 0) + (o[2] != 0) <= 1;
     }
-    op->general = range <= 6 && (!cfd || axis_aligned);
+    op->general = !force_generic && range <= 6 && (!cfd || axis_aligned);
     *out = op;
     return 0;
 }

@@ -38,3 +38,21 @@ def test_axis_order(nn):
     assert _path(_axes((2, 1, 0), nn)) == TILED
     for order in [(0, 1, 2), (2, 0, 1), (1, 2, 0)]:
         assert _path(_axes(order, nn)) == GENERAL
+
+
+def test_generic_path_on_request(monkeypatch):
+    """GPAW_B200_FD_PATH=generic: one thread a point for every stencil, so
+    that the other kernels can be compared with it."""
+    skew = [(0, 0, 0), (1, -1, 0), (-1, 1, 0), (0, 2, 1)]
+    assert _path(skew) == GENERAL
+    monkeypatch.setenv('GPAW_B200_FD_PATH', 'generic')
+    assert _path(skew) == GENERIC
+    assert _path(_axes((2, 1, 0), 3)) == GENERIC
+
+
+def test_stencils_left_to_the_generic_path():
+    """Ranges above 6, and diagonal taps declared axis-aligned (their corner
+    values read zero)."""
+    assert _path([(0, 0, 0), (7, -1, 0)]) == GENERIC
+    assert _path([(0, 0, 0), (1, 1, 0)], cfd=True) == GENERIC
+    assert _path([(0, 0, 0), (1, 1, 0)], cfd=False) == GENERAL

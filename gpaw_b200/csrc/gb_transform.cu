@@ -1164,15 +1164,18 @@ k_density_sums(const double* __restrict__ n, const double* __restrict__ w0,
     }
 }
 
-// scale = coarse integral / fine integral where the latter exceeds 1e-14
+// scale = coarse integral / fine integral where the latter exceeds 1e-14.
+// Above order 2 the interpolation weights have both signs, so an infinite
+// coarse value makes the sum over the fine grid NaN, which leaves the density
+// as it is; here the weighted sum stays infinite.
 __global__ void __launch_bounds__(DENSITY_BLOCKS)
-k_density_scale(const double* __restrict__ partial, double dv, double dvf,
+k_density_scale(const double* __restrict__ partial, int k, double dv, double dvf,
                 double* __restrict__ scale) {
     const double s = block_sum(partial[2 * (blockIdx.x * DENSITY_BLOCKS + threadIdx.x)]);
     const double w = block_sum(partial[2 * (blockIdx.x * DENSITY_BLOCKS + threadIdx.x) + 1]);
     if (threadIdx.x == 0) {
         const double a = s * dv, b = w * dvf;
-        scale[blockIdx.x] = b > 1e-14 ? a / b : 1.0;
+        scale[blockIdx.x] = b > 1e-14 && (k == 2 || isfinite(b)) ? a / b : 1.0;
     }
 }
 
@@ -1185,7 +1188,7 @@ int launch_density(int k, const double* in, double* out, int nin, const XferGeom
     double* scale = work + (size_t)nin * 2 * DENSITY_BLOCKS;
     k_density_sums<<<dim3(DENSITY_BLOCKS, nin), 256, 0, st>>>(
         in, w[0], w[1], w[2], G.g.n[0], G.g.n[1], G.g.n[2], work);
-    k_density_scale<<<nin, DENSITY_BLOCKS, 0, st>>>(work, dv, dvf, scale);
+    k_density_scale<<<nin, DENSITY_BLOCKS, 0, st>>>(work, k, dv, dvf, scale);
     const Phases P{};
     switch (k) {
         case 2: return launch_interp_v<double, 2, 0>(in, out, nin, G, P, st, scale);

@@ -485,7 +485,6 @@ int DirectTables::build(const GridBC& g, const double* const pe[3], const double
 DirectGroup::~DirectGroup() {
     if (exec) cudaGraphExecDestroy(exec);
     dfree(mem);
-    if (ctl_host) hfree(ctl_host);
 }
 
 int DirectGroup::build(const std::vector<DirGrid>& desc, int half_width, cudaStream_t cs) {
@@ -536,7 +535,9 @@ int DirectGroup::build(const std::vector<DirGrid>& desc, int half_width, cudaStr
     size_t size = off_part + al(npart * sizeof(double));
     for (auto& m : maps) size += al(m.second.size() * sizeof(DirBlock));
     GB_CUDA_TRY(pool_malloc(&mem, size));
-    GB_CUDA_TRY(pool_malloc_host(&ctl_host, n * sizeof(DirCtl)));
+    DirCtl* host = nullptr;
+    GB_CUDA_TRY(pool_malloc_host(&host, n * sizeof(DirCtl)));
+    results.reset(host, [](DirCtl* p) { hfree(p); });
     grids = (DirGrid*)mem;
     ctl = (DirCtl*)(mem + off_ctl);
     for (int i = 0; i < n; i++) d[i].partial = (double*)(mem + off_part) + psum[i];
@@ -605,7 +606,8 @@ int DirectGroup::capture(cudaStream_t cs) {
 
 int DirectGroup::run(cudaStream_t st) {
     GB_CUDA_TRY(cudaGraphLaunch(exec, st));
-    GB_CUDA_TRY(cudaMemcpyAsync(ctl_host, ctl, n * sizeof(DirCtl), cudaMemcpyDeviceToHost, st));
+    GB_CUDA_TRY(cudaMemcpyAsync(results.get(), ctl, n * sizeof(DirCtl), cudaMemcpyDeviceToHost,
+                                st));
     return 0;
 }
 

@@ -2,6 +2,7 @@
 // of one solver, and a group of grids solved by one captured loop.
 #pragma once
 
+#include <memory>
 #include <vector>
 
 #include "gb_direct.cuh"
@@ -23,7 +24,8 @@ struct DirectGroup {
     char* mem = nullptr;
     DirGrid* grids = nullptr;
     DirCtl* ctl = nullptr;
-    DirCtl* ctl_host = nullptr;
+    // outcomes of the last launch, one a grid (pinned); solvers share them
+    std::shared_ptr<DirCtl> results;
     // the CTAs of one launch: grids of one block shape along one axis
     struct Part {
         DirBlock* map = nullptr;   // (one grid: block index alone)

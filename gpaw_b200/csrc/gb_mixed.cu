@@ -22,6 +22,7 @@
 #include <cstdlib>
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <utility>
 #include <vector>
 
@@ -727,7 +728,9 @@ struct gb_mixed {
     // separable: its tables, and this solver as a group of one
     DirectTables* dtab = nullptr;
     DirectGroup* dgrp = nullptr;
-    const DirCtl* dres = nullptr;      // outcome of the last solve, if direct (pinned)
+    // outcome of the last solve, if direct: a share of its group's results,
+    // so that solvers and groups may be freed in any order
+    std::shared_ptr<const DirCtl> dres;
     ~gb_mixed() {
         delete dgrp;
         delete dtab;
@@ -1597,7 +1600,7 @@ extern "C" int gb_mixed_solve_async(gb_mixed* m, double* phi, const double* rho,
     if (m->dtab && maxiter >= DIRECT_MIN_MAXITER) {
         if (!m->dgrp)
             if (int rc = build_direct_group(m)) return rc;
-        m->dres = m->dgrp->ctl_host;
+        m->dres = m->dgrp->results;
         if (ranges_overlap(phi, rho, bytes)) {
             // phi changes while rho is still read: a copy of rho
             GB_CUDA_TRY(cudaMemcpyAsync(m->rho0, rho, bytes, cudaMemcpyDeviceToDevice, st));
@@ -1622,13 +1625,10 @@ extern "C" int gb_mixed_solve_async(gb_mixed* m, double* phi, const double* rho,
 
 extern "C" int gb_mixed_result(gb_mixed* m, int* niter, double* rel_residual) {
     if (!m) return fail(GB_EINVAL, "mixed result: NULL solver");
-    if (m->dres) {
-        m->ctl_host->niter = m->dres->niter;
-        m->ctl_host->rel = m->dres->rel;
-    }
-    if (niter) *niter = m->ctl_host->niter;
-    if (rel_residual) *rel_residual = m->ctl_host->rel;
-    if (m->ctl_host->rel > m->last_tol)
+    const double rel = m->dres ? m->dres->rel : m->ctl_host->rel;
+    if (niter) *niter = m->dres ? m->dres->niter : m->ctl_host->niter;
+    if (rel_residual) *rel_residual = rel;
+    if (rel > m->last_tol)
         return fail(GB_ENOCONV, "mixed-precision Poisson solver did not reach %g in %d V-cycles",
                     m->last_tol, m->last_maxiter);
     return 0;
@@ -1680,12 +1680,6 @@ struct gb_mixed_batch {
     cudaGraphExec_t exec = nullptr;
     DirectGroup* dgrp = nullptr;   // every grid by the direct correction
     ~gb_mixed_batch() {
-        for (int i = 0; i < n && dgrp; i++)     // results outlive the batch
-            if (s[i]->dres == dgrp->ctl_host + i) {
-                s[i]->ctl_host->niter = s[i]->dres->niter;
-                s[i]->ctl_host->rel = s[i]->dres->rel;
-                s[i]->dres = nullptr;
-            }
         delete dgrp;
         if (exec) cudaGraphExecDestroy(exec);
         if (cap) cudaStreamDestroy(cap);
@@ -1919,7 +1913,9 @@ extern "C" int gb_mixed_batch_solve_async(gb_mixed_batch* bt, double* const* phi
         bt->h_user[2 * i + 1] = const_cast<double*>(rhos[i]);
         bt->s[i]->last_tol = bt->tol;
         bt->s[i]->last_maxiter = bt->maxiter;
-        bt->s[i]->dres = bt->dgrp ? bt->dgrp->ctl_host + i : nullptr;
+        bt->s[i]->dres.reset();
+        if (bt->dgrp)
+            bt->s[i]->dres = {bt->dgrp->results, bt->dgrp->results.get() + i};
     }
     if (bt->dgrp && batch_overlaps(bt))
         // some phi changes while a rho that it shares memory with is still
@@ -1941,14 +1937,12 @@ extern "C" int gb_mixed_batch_result(gb_mixed_batch* bt, int* niters, double* re
     if (!bt) return fail(GB_EINVAL, "mixed batch result: NULL batch");
     int bad = -1;
     for (int i = 0; i < bt->n; i++) {
-        Ctl* c = bt->s[i]->ctl_host;
-        if (bt->dgrp) {
-            c->niter = bt->dgrp->ctl_host[i].niter;
-            c->rel = bt->dgrp->ctl_host[i].rel;
-        }
-        if (niters) niters[i] = c->niter;
-        if (rel_residuals) rel_residuals[i] = c->rel;
-        if (c->rel > bt->tol && bad < 0) bad = i;
+        const Ctl* c = bt->s[i]->ctl_host;
+        const DirCtl* d = bt->dgrp ? bt->dgrp->results.get() + i : nullptr;
+        const double rel = d ? d->rel : c->rel;
+        if (niters) niters[i] = d ? d->niter : c->niter;
+        if (rel_residuals) rel_residuals[i] = rel;
+        if (rel > bt->tol && bad < 0) bad = i;
     }
     if (bad >= 0)
         return fail(GB_ENOCONV, "mixed batch: solve %d did not reach %g in %d V-cycles", bad,

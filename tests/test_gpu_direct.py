@@ -105,3 +105,35 @@ def test_direct_phi_may_be_rho(cuda):
     batch.solve([c, d], [c, c])
     assert torch.equal(c, a)
     assert _residual(gdo, 3, to_np(d), to_np(rho)) <= 1.01e-10
+
+
+def test_batch_and_solvers_freed_in_any_order(cuda):
+    """A solver keeps its outcome when the batch is gone, and the batch may
+    be the last to go."""
+    import gc
+    import torch
+    from gpaw_b200 import GridDescriptor
+    from gpaw_b200.batch import PoissonBatch
+    gds = [GridDescriptor(N, 4.0, 0) for N in ((16, 24, 32), (24, 16, 16))]
+    rng = np.random.default_rng(5)
+    rhos = [to_dev(rng.standard_normal(tuple(gd.n_c))) for gd in gds]
+
+    def solved():
+        batch = PoissonBatch(gds)
+        batch.enqueue([gd.zeros() for gd in gds], rhos)
+        torch.cuda.synchronize()
+        return batch
+
+    batch = solved()
+    want = batch.results()
+    solvers = batch.solvers
+    del batch
+    gc.collect()
+    assert [ps.result() for ps in solvers] == want
+    assert all(0 < ps.rel_residual <= 1e-10 for ps in solvers)
+    batch = solved()
+    for ps in batch.solvers:
+        ps._h = None                  # frees the solver
+    gc.collect()
+    del batch
+    gc.collect()

@@ -296,7 +296,8 @@ class _CoarseLevels:
             if int(np.prod(solver.operators[first].gd.n_c)) <= 32768 and \
                     solver.levels - first + 1 <= cls.MAX_LEVELS:
                 obj = cls(solver, first)
-                return obj if obj._h.value else None
+                if obj._h.value:
+                    return obj
         return None
 
     def __init__(self, solver, first):

@@ -247,6 +247,7 @@ k_direct(const DirGrid* __restrict__ grids, const DirCtl* ctl, const DirBlock* _
             }
             __syncthreads();
             if (has_e) put(S, DIR_P, ke, he);
+            __syncthreads();    // the odd half's padding reads even rows (times zero)
             if (has_o) {
                 product(acc, oa, kpo, SO, -DIR_P, ring, lane);
                 if (div) divide(ax.lam + he, ko, ho);

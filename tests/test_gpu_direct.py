@@ -137,3 +137,26 @@ def test_batch_and_solvers_freed_in_any_order(cuda):
     gc.collect()
     del batch
     gc.collect()
+
+
+@pytest.mark.parametrize('N,pbc', [((192, 16, 24), 0), ((16, 190, 24), 1),
+                                   ((16, 24, 100), 0)])
+def test_direct_is_deterministic_for_any_data(N, pbc, cuda):
+    """Sums that overflow or are not finite: the same outcome every time (a
+    half of an axis reads no row that another warp writes)."""
+    gd, ps, gdo = _solver(N, pbc)
+    rng = np.random.default_rng(6)
+    for bad in (1e308, np.inf, np.nan):
+        rho = rng.standard_normal(tuple(gdo.n_c))
+        rho[tuple(n // 3 for n in rho.shape)] = bad
+        seen = []
+        for _ in range(4):
+            phi = gd.zeros()
+            try:
+                ps.solve_neutral(phi, to_dev(rho))
+            except RuntimeError:
+                pass
+            seen.append((ps.niter, to_np(phi)))
+        for n, phi in seen[1:]:
+            assert n == seen[0][0]
+            assert np.array_equal(phi, seen[0][1], equal_nan=True)

@@ -4,10 +4,12 @@ one GPU.
 Each grid gets its own solver: its own device-resident level hierarchy,
 buffers and captured V-cycle loop (the whole solve runs on the device, see
 gb_poisson_* / gb_mixed_*).  A mixed batch is, by default, ONE CUDA graph
-(gb_mixed_batch_*): with the direct correction each kernel works on every
-grid at once, with V-cycles the graph has a branch per grid.  Otherwise (FP64, or graph=False)
-the batch enqueues every solve on one of ``nstreams`` CUDA streams.  Either
-way there is no host synchronisation until the results are read.
+(gb_mixed_batch_*): with the direct correction (``correction`` as in
+MixedPoissonSolver; 'auto' takes it when every grid has one) each kernel works
+on every grid at once, with V-cycles the graph has a branch per grid.
+Otherwise (FP64, or graph=False) the batch enqueues every solve on one of
+``nstreams`` CUDA streams.  Either way there is no host synchronisation until
+the results are read.
 """
 from __future__ import annotations
 
@@ -23,7 +25,7 @@ from .poisson import FDPoissonSolver, MixedPoissonSolver
 
 class PoissonBatch:
     def __init__(self, gds, nn=3, tol=1e-10, precision='mixed', nstreams=16,
-                 maxiter=400, levels=4, graph=True):
+                 maxiter=400, levels=4, graph=True, correction='auto'):
         if precision not in ('mixed', 'fp64'):
             raise ValueError("precision must be 'mixed' or 'fp64'")
         self.gds = list(gds)
@@ -33,7 +35,7 @@ class PoissonBatch:
         # hundreds of solvers are built at once: through the library's
         # caching allocator, which carves their buffers from a few slabs
         with solver_pool():
-            self._build(nn, tol, maxiter, levels, precision)
+            self._build(nn, tol, maxiter, levels, precision, correction)
         dev = self.gds[0].device if self.gds else torch.device('cuda')
         self.streams = [torch.cuda.Stream(device=dev)
                         for _ in range(max(1, nstreams))]
@@ -47,14 +49,15 @@ class PoissonBatch:
                                          int(maxiter), C.byref(h)))
             self._batch = (lib, h)
 
-    def _build(self, nn, tol, maxiter, levels, precision):
+    def _build(self, nn, tol, maxiter, levels, precision, correction):
         for gd in self.gds:
             if precision == 'mixed':
                 # the coarse levels in one single-block kernel a solve: the
                 # batch's solves run side by side, which cooperative kernels
                 # (the whole GPU at once) would serialise
                 ps = MixedPoissonSolver(nn=nn, tol=tol, maxiter=maxiter,
-                                        levels=levels, fused_coarse='tail')
+                                        levels=levels, fused_coarse='tail',
+                                        correction=correction)
             else:
                 ps = FDPoissonSolver(nn=nn, relax='J', eps=0.0,
                                      maxiter=maxiter)

@@ -727,6 +727,7 @@ struct gb_mixed {
     // the direct correction (gb_direct.cu), where the level-0 operator is
     // separable: its tables, and this solver as a group of one
     DirectTables* dtab = nullptr;
+    int correction = 0;       // gb_mixed_set_correction
     DirectGroup* dgrp = nullptr;
     // outcome of the last solve, if direct: a share of its group's results,
     // so that solvers and groups may be freed in any order
@@ -1502,11 +1503,15 @@ static int build_mixed_graph(gb_mixed* m) {
 static int prepare_vcycles(gb_mixed* m);
 
 // --------------------------------------------------------- direct correction
-// Solves that allow at least this many V-cycles take the direct correction
-// where the grid has one.  V-cycle counts measured on every grid shape of
-// the benchmarks and tests are 10 to 23; a caller who allows fewer than 50
-// may be asking to be stopped, and is: such a solve keeps the V-cycles.
+// The automatic choice: solves that allow at least this many V-cycles take
+// the direct correction where the grid has one.  V-cycle counts measured on
+// every grid shape of the benchmarks and tests are 10 to 23, so a lower limit
+// may be there to stop the solve, and does: it keeps the V-cycles.
 constexpr int DIRECT_MIN_MAXITER = 50;
+
+static bool takes_direct(const gb_mixed* m, int maxiter) {
+    return m->dtab && m->correction != 2 && (m->correction == 1 || maxiter >= DIRECT_MIN_MAXITER);
+}
 
 static DirGrid direct_desc(const gb_mixed* m) {
     DirGrid d{};
@@ -1564,6 +1569,16 @@ extern "C" int gb_mixed_set_direct(gb_mixed* m, const double* const* pe, const d
     return 0;
 }
 
+extern "C" int gb_mixed_set_correction(gb_mixed* m, int correction) {
+    if (!m) return fail(GB_EINVAL, "mixed: NULL solver");
+    if (correction < 0 || correction > 2)
+        return fail(GB_EINVAL, "mixed: correction must be 0, 1 or 2");
+    if (correction == 1 && !m->dtab)
+        return fail(GB_EINVAL, "mixed: this solver has no direct correction");
+    m->correction = correction;
+    return 0;
+}
+
 extern "C" int gb_mixed_prepare(gb_mixed* m) {
     if (!m) return fail(GB_EINVAL, "mixed prepare: NULL solver");
     if (m->dtab) {
@@ -1597,7 +1612,7 @@ extern "C" int gb_mixed_solve_async(gb_mixed* m, double* phi, const double* rho,
     const size_t bytes = (size_t)n * sizeof(double);
     m->last_tol = tol;
     m->last_maxiter = maxiter;
-    if (m->dtab && maxiter >= DIRECT_MIN_MAXITER) {
+    if (takes_direct(m, maxiter)) {
         if (!m->dgrp)
             if (int rc = build_direct_group(m)) return rc;
         m->dres = m->dgrp->results;
@@ -1872,11 +1887,17 @@ extern "C" int gb_mixed_batch_new(int n, gb_mixed* const* solvers, double tol, i
             if (solvers[j] == solvers[i])
                 return fail(GB_EINVAL, "mixed batch: solver %d appears twice", i);
     }
-    // the direct path when every grid has one (and the same half-width, which
-    // the grouped defect kernel is compiled for)
-    bool direct = maxiter >= DIRECT_MIN_MAXITER;
-    for (int i = 0; i < n; i++)
-        direct = direct && solvers[i]->dtab && solvers[i]->op64->nn == solvers[0]->op64->nn;
+    // the direct path when every solver takes it (and has the same half-width,
+    // which the grouped defect kernel is compiled for)
+    bool direct = true, asked = false;
+    for (int i = 0; i < n; i++) {
+        direct = direct && takes_direct(solvers[i], maxiter) &&
+                 solvers[i]->op64->nn == solvers[0]->op64->nn;
+        asked = asked || solvers[i]->correction == 1;
+    }
+    if (asked && !direct)
+        return fail(GB_EINVAL, "mixed batch: a solver asks for the direct correction, which the "
+                               "batch cannot take for every grid");
     // one uncaptured pass of every kernel (sets kernel attributes)
     for (int i = 0; i < n && !direct; i++)
         if (!solvers[i]->exec)

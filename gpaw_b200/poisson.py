@@ -433,12 +433,20 @@ class MixedPoissonSolver:
     residual, its norm, |rho| and the stopping test
     ||rho - L phi|| <= tol ||rho|| are FP64, on the device.
 
-    Corrections: where the level-0 operator is a sum of axis stencils (up to
-    384 points a side) and at least 50 V-cycles are allowed, by fast
-    diagonalisation in FP64 (the eigenvectors of each axis, see
-    gpaw_b200.separable), which solves to rounding: one correction, 0.75 ms
-    on a 192^3 grid, against 14 V-cycles and 5.35 ms.  Otherwise by FP32
-    V-cycles over ``levels`` grids (fewer when the grid cannot be coarsened
+    Corrections, as ``correction`` says:
+
+    'direct'  by fast diagonalisation in FP64 (the eigenvectors of each axis,
+              see gpaw_b200.separable), which solves to rounding: one
+              correction, 0.75 ms on a 192^3 grid, against 14 V-cycles and
+              5.35 ms.  For level-0 operators that are a sum of axis stencils
+              (nn up to 3, up to 384 points a side); ValueError for others.
+              ``levels`` and ``fused_coarse`` have no effect.
+    'vcycle'  by FP32 V-cycles.
+    'auto'    (the default) 'direct' where it is possible and ``maxiter`` is
+              at least 50, else 'vcycle': a lower limit is taken as one on
+              V-cycles, of which a solve needs 10 to 23.
+
+    V-cycles span ``levels`` grids (fewer when the grid cannot be coarsened
     that often) with degree-2 Chebyshev smoothing (two sweeps before, two
     after); the coarsest grid is solved in FP64: by default exactly, by fast
     diagonalisation in one cooperative kernel over every SM; with
@@ -450,16 +458,20 @@ class MixedPoissonSolver:
     """
 
     def __init__(self, nn=3, tol=1e-10, maxiter=200, levels=6,
-                 coarse_accuracy=0.2, fused_coarse=True):
+                 coarse_accuracy=0.2, fused_coarse=True, correction='auto'):
         if nn == 'M':
             raise NotImplementedError(
                 'Mehrstellen stencil: use FDPoissonSolver(nn="M")')
+        if correction not in ('auto', 'direct', 'vcycle'):
+            raise ValueError("correction must be 'auto', 'direct' or "
+                             "'vcycle'")
         self.nn = nn
         self.tol = tol
         self.maxiter = maxiter
         self.nlevels = levels
         self.coarse_accuracy = coarse_accuracy
         self.fused_coarse = fused_coarse
+        self.correction = correction
         self._h = None
 
     def set_grid_descriptor(self, gd):
@@ -506,12 +518,16 @@ class MixedPoissonSolver:
                                itp, lam, float(self.lam_min_coarse),
                                int(self.coarse_degree), C.byref(h)))
         self._h = _MixedHandle(lib, h, self)
-        modes = separable_modes(self.operators[0], gd)
+        modes = None
+        if self.correction != 'vcycle':
+            modes = separable_modes(self.operators[0], gd)
         if modes is not None:
             dp = C.POINTER(C.c_double)
             arg = [(dp * 3)(*[m[k].ctypes.data_as(dp) for m in modes])
                    for k in range(3)]
             check(lib.gb_mixed_set_direct(h, *arg))
+        if self.correction == 'direct':
+            check(lib.gb_mixed_set_correction(h, 1))
         mode = 2 if self.fused_coarse == 'tail' else int(bool(self.fused_coarse))
         check(lib.gb_mixed_set_fused_coarse(h, mode))
 

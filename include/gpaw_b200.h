@@ -364,15 +364,23 @@ GB_API int gb_mixed_set_fused_coarse(gb_mixed* m, int mode);
  * h = (n + 1) / 2 (zero) or n / 2 + 1 (periodic) for the points 0 .. h - 1,
  * po[a] the same for the n - h points that have a distinct mirror point;
  * columns of unit norm over all n points.  lam[a]: n eigenvalues, even first;
- * their sum over the axes is the operator's eigenvalue.  Solves that allow at least 50
- * V-cycles then correct phi by e = L^-1 d in FP64 (fast diagonalisation)
- * instead of an FP32 V-cycle, inside the same defect-correction loop;
- * V-cycle counts become counts of corrections (one or two).  A grid the path
- * does not take (stencils wider than 3, more than 384 points a side,
- * unsymmetric coefficients) keeps the V-cycles; returns 0 either way.  Call
- * it once, before the first solve.  No counterpart in the reference. */
+ * their sum over the axes is the operator's eigenvalue.  Solves can
+ * then correct phi by e = L^-1 d in FP64 (fast diagonalisation) instead of an
+ * FP32 V-cycle, inside the same defect-correction loop (which solves do:
+ * gb_mixed_set_correction); V-cycle counts become counts of corrections (one
+ * or two).  A grid the path does not take (stencils wider than 3, more than
+ * 384 points a side, unsymmetric coefficients) keeps the V-cycles; returns 0
+ * either way.  Call it once, before the first solve.  No counterpart in the
+ * reference. */
 GB_API int gb_mixed_set_direct(gb_mixed* m, const double* const* pe, const double* const* po,
                                const double* const* lam);
+/* Which correction a solve uses: 0 (the default) the direct one where the
+ * solver has it and at least 50 corrections are allowed, else V-cycles; 1 the
+ * direct one (GB_EINVAL where the solver has none); 2 V-cycles.  A batch uses
+ * one kind for all its solvers, as they stand when it is made: the direct one
+ * when each of them would; GB_EINVAL when one asks for it by 1 and another
+ * would not.  No counterpart in the reference. */
+GB_API int gb_mixed_set_correction(gb_mixed* m, int correction);
 /* One V-cycle of the mixed-precision solver and the defects around it,
  * launched kernel by kernel instead of through the solver's graph:
  * phi <- phi + V32(rho - L phi).  For profilers and kernel traces (its

@@ -24,7 +24,8 @@ def _rhos(gds):
             for i, gd in enumerate(gds)]
 
 
-def test_graph_batch_equals_streams_and_single(cuda):
+@pytest.mark.parametrize('correction', ['vcycle', 'auto'])
+def test_graph_batch_equals_streams_and_single(correction, cuda):
     from gpaw_b200 import MixedPoissonSolver
     from gpaw_b200.batch import PoissonBatch
     gds = _grids()
@@ -32,31 +33,55 @@ def test_graph_batch_equals_streams_and_single(cuda):
     out = {}
     for mode in ('graph', 'streams'):
         b = PoissonBatch(gds, tol=1e-10, precision='mixed',
-                         graph=(mode == 'graph'), nstreams=4)
+                         graph=(mode == 'graph'), nstreams=4,
+                         correction=correction)
         phis = [gd.zeros() for gd in gds]
         n = b.solve(phis, rhos)
         out[mode] = (n, [to_np(p) for p in phis])
         # a second call on the same batch reuses the graph
         phis2 = [gd.zeros() for gd in gds]
         assert b.solve(phis2, rhos) == n
+        assert min(n) > 5 if correction == 'vcycle' else max(n) <= 2
         for p, q in zip(phis, phis2):
             assert np.array_equal(to_np(p), to_np(q))
     assert out['graph'][0] == out['streams'][0]
     for p, q in zip(out['graph'][1], out['streams'][1]):
         assert np.array_equal(p, q)
     # one solver alone
-    ps = MixedPoissonSolver(tol=1e-10, maxiter=400, fused_coarse='tail')
+    ps = MixedPoissonSolver(tol=1e-10, maxiter=400, fused_coarse='tail',
+                            correction=correction)
     ps.set_grid_descriptor(gds[2])
     phi = gds[2].zeros()
     ps.solve_neutral(phi, rhos[2])
     assert np.array_equal(to_np(phi), out['graph'][1][2])
 
 
-def test_graph_batch_against_reference(cuda):
+def test_one_grid_without_a_direct_correction(cuda):
+    """A side above 384 points: that batch solves every grid by V-cycles."""
+    from gpaw_b200 import GridDescriptor
+    from gpaw_b200.batch import PoissonBatch
+    gds = _grids()[:3] + [GridDescriptor((400, 16, 24), (80.0, 3.2, 4.8), 0)]
+    rhos = _rhos(gds)
+    b = PoissonBatch(gds, tol=1e-10)
+    phis = [gd.zeros() for gd in gds]
+    n = b.solve(phis, rhos)
+    assert min(n) > 5
+    for gd, rho, phi in zip(gds, rhos, phis):
+        gref = L.GridDescriptor(tuple(gd.N_c), gd.cell_cv, tuple(gd.pbc_c))
+        got = np.zeros(tuple(gd.n_c))
+        L.Laplace(gref, -0.25 / np.pi, 3).apply(to_np(phi), got)
+        rho = to_np(rho)
+        assert np.linalg.norm(rho - got) <= 1.01e-10 * np.linalg.norm(rho)
+    with pytest.raises(ValueError, match='direct'):
+        PoissonBatch(gds, correction='direct')
+
+
+@pytest.mark.parametrize('correction', ['vcycle', 'auto'])
+def test_graph_batch_against_reference(correction, cuda):
     from gpaw_b200.batch import PoissonBatch
     gds = _grids()[:3]
     rhos = _rhos(gds)
-    b = PoissonBatch(gds, tol=1e-11, precision='mixed')
+    b = PoissonBatch(gds, tol=1e-11, precision='mixed', correction=correction)
     phis = [gd.zeros() for gd in gds]
     b.solve(phis, rhos)
     for gd, rho, phi in zip(gds, rhos, phis):

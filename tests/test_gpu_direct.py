@@ -72,6 +72,22 @@ def test_direct_against_dense_solution(pbc, cuda):
     assert np.linalg.norm(to_np(phi) - ref) <= 1e-10 * np.linalg.norm(ref)
 
 
+def test_the_caller_chooses_the_correction(cuda):
+    """Direct under a low limit, V-cycles under a high one; a grid without a
+    direct correction is refused."""
+    N = (48, 40, 56)
+    for correction, maxiter in (('direct', 2), ('vcycle', 200)):
+        gd, ps, gdo = _solver(N, 0, maxiter=maxiter, correction=correction)
+        rho = np.random.default_rng(3).standard_normal(tuple(gdo.n_c))
+        phi = gd.zeros()
+        n = ps.solve_neutral(phi, to_dev(rho))
+        assert (n > 5) == (correction == 'vcycle')
+        assert _residual(gdo, 3, to_np(phi), rho) <= 1.01e-10
+    for N, nn in (((8, 16, 386), 3), ((16, 16, 16), 4)):
+        with pytest.raises(ValueError, match='direct'):
+            _solver(N, 0, nn, correction='direct')
+
+
 def test_few_vcycles_allowed_keeps_the_vcycles(cuda):
     """maxiter below 50 is a limit on V-cycles: that path, same solution."""
     N = (48, 40, 56)

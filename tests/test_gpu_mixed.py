@@ -1,11 +1,13 @@
-"""Mixed-precision Poisson solver (FP32 V-cycles in FP64 defect correction)
-against the FP64 oracle.
+"""Mixed Poisson solver (FP64 defect correction, by FP32 V-cycles in each form
+of their coarse levels and by the direct correction) against the FP64 oracle.
 
 Bar: the relative residual ||rho - L phi|| / ||rho||, recomputed here in
 FP64 by the oracle's own operator, is at most 1e-10 (x 1.01 for the
 different summation order), and the potential agrees with the oracle's FP64
 solution (solved to 1e-12) within 1e-7 relative (max norm); the measured
 maximum error is printed."""
+import functools
+
 import numpy as np
 import pytest
 
@@ -23,17 +25,33 @@ def _case(N, pbc, seed):
     return gdo, rho
 
 
-@pytest.mark.parametrize('fused', [True, False, 'tail'])
+@functools.lru_cache(maxsize=None)
+def _oracle_solution(N, pbc, seed):
+    """The oracle's FP64 solution to 1e-12 relative."""
+    gdo, rho = _case(N, pbc, seed)
+    eps = (1e-12 * np.sqrt((rho * rho).sum()))**2 * gdo.dv
+    po = L.FDPoissonSolver(nn=3, eps=eps, maxiter=2000)
+    po.set_grid_descriptor(gdo)
+    ref = gdo.zeros()
+    po.solve_neutral(ref, rho)
+    return ref
+
+
+@pytest.mark.parametrize('correction,fused', [
+    ('vcycle', True), ('vcycle', False), ('vcycle', 'tail'), ('auto', True)])
 @pytest.mark.parametrize('N,pbc', [((64, 64, 64), 0), ((48, 40, 56), 0),
                                    ((48, 48, 48), 1)])
-def test_mixed_reaches_1e10_and_matches_fp64(N, pbc, fused, cuda, capsys):
-    """Both forms of the coarse levels (one cooperative kernel with the
-    exact coarsest solve, or one kernel a pass with the Chebyshev coarsest
-    solve) reach the tolerance and the FP64 solution."""
+def test_mixed_reaches_1e10_and_matches_fp64(N, pbc, correction, fused, cuda,
+                                             capsys):
+    """Every form of the coarse levels (one cooperative kernel with the exact
+    coarsest solve, one kernel a pass with the Chebyshev coarsest solve, one
+    single-block kernel) and the direct correction reach the tolerance and
+    the FP64 solution."""
     from gpaw_b200 import GridDescriptor, MixedPoissonSolver
     gdo, rho = _case(N, pbc, seed=3)
     gdp = GridDescriptor(N, np.diag(gdo.cell_cv), pbc)
-    ps = MixedPoissonSolver(nn=3, tol=1e-10, fused_coarse=fused)
+    ps = MixedPoissonSolver(nn=3, tol=1e-10, fused_coarse=fused,
+                            correction=correction)
     ps.set_grid_descriptor(gdp)
     phi = gdp.zeros()
     n = ps.solve_neutral(phi, to_dev(rho))
@@ -43,21 +61,17 @@ def test_mixed_reaches_1e10_and_matches_fp64(N, pbc, fused, cuda, capsys):
     lphi = np.zeros_like(got)
     op.apply(got, lphi)
     rel = np.sqrt(((rho - lphi)**2).sum() / (rho**2).sum())
-    # oracle FP64 solution to 1e-12 relative
-    eps = (1e-12 * np.sqrt((rho * rho).sum()))**2 * gdo.dv
-    po = L.FDPoissonSolver(nn=3, eps=eps, maxiter=2000)
-    po.set_grid_descriptor(gdo)
-    ref = gdo.zeros()
-    po.solve_neutral(ref, rho)
+    ref = _oracle_solution(N, pbc, 3)
     err = np.abs(got - ref).max() / np.abs(ref).max()
     with capsys.disabled():
-        print(f'\nmixed {N} pbc={pbc} fused={fused}: {n} V-cycles, '
+        print(f'\nmixed {N} pbc={pbc} {correction} fused={fused}: '
+              f'{n} corrections, '
               f'rel residual {rel:.3e} '
               f'(device {ps.rel_residual:.3e}), max rel error vs FP64 '
               f'{err:.3e}')
     assert rel <= 1.01e-10
     assert err <= 1e-7
-    assert n < 40
+    assert 5 < n < 40 if correction == 'vcycle' else n <= 2
 
 
 def test_mixed_nonconvergence_raises(cuda):

@@ -49,6 +49,8 @@ SIGNATURES = {
                                 C.POINTER(C.c_size_t)]),
     'gb_mixed_set_direct': (C.c_int, [_p, C.POINTER(_dp), C.POINTER(_dp),
                                       C.POINTER(_dp)]),
+    'gb_mixed_prepare_for': (C.c_int, [_p, C.c_int]),
+    'gb_mixed_prepared': (C.c_int, [_p, C.c_int]),
     'gb_mixed_set_correction': (C.c_int, [_p, C.c_int]),
     'gb_mixed_vcycle_eager': (C.c_int, [_p, _p, _p, _p]),
     'gb_mixed_set_fused_coarse': (C.c_int, [_p, C.c_int]),

@@ -1581,11 +1581,20 @@ extern "C" int gb_mixed_set_correction(gb_mixed* m, int correction) {
 
 extern "C" int gb_mixed_prepare(gb_mixed* m) {
     if (!m) return fail(GB_EINVAL, "mixed prepare: NULL solver");
-    if (m->dtab) {
-        if (!m->dgrp) return build_direct_group(m);
-        return 0;
-    }
-    return prepare_vcycles(m);
+    // whatever limit a solve will have
+    if (int rc = gb_mixed_prepare_for(m, 1)) return rc;
+    return gb_mixed_prepare_for(m, DIRECT_MIN_MAXITER);
+}
+
+extern "C" int gb_mixed_prepare_for(gb_mixed* m, int maxiter) {
+    if (!m) return fail(GB_EINVAL, "mixed prepare: NULL solver");
+    if (!takes_direct(m, maxiter)) return prepare_vcycles(m);
+    return m->dgrp ? 0 : build_direct_group(m);
+}
+
+extern "C" int gb_mixed_prepared(const gb_mixed* m, int maxiter) {
+    if (!m) return 0;
+    return takes_direct(m, maxiter) ? m->dgrp != nullptr : m->exec != nullptr;
 }
 
 static int prepare_vcycles(gb_mixed* m) {
@@ -1613,8 +1622,7 @@ extern "C" int gb_mixed_solve_async(gb_mixed* m, double* phi, const double* rho,
     m->last_tol = tol;
     m->last_maxiter = maxiter;
     if (takes_direct(m, maxiter)) {
-        if (!m->dgrp)
-            if (int rc = build_direct_group(m)) return rc;
+        if (int rc = gb_mixed_prepare_for(m, maxiter)) return rc;
         m->dres = m->dgrp->results;
         if (ranges_overlap(phi, rho, bytes)) {
             // phi changes while rho is still read: a copy of rho
@@ -1624,7 +1632,7 @@ extern "C" int gb_mixed_solve_async(gb_mixed* m, double* phi, const double* rho,
         return m->dgrp->solve(phi, rho, tol, maxiter, st);
     }
     m->dres = nullptr;
-    if (int rc = prepare_vcycles(m)) return rc;
+    if (int rc = gb_mixed_prepare_for(m, maxiter)) return rc;
     GB_CUDA_TRY(cudaMemcpyAsync(m->rho0, rho, bytes, cudaMemcpyDeviceToDevice, st));
     GB_CUDA_TRY(cudaMemcpyAsync(m->phi0, phi, bytes, cudaMemcpyDeviceToDevice, st));
     const int nb = (int)std::min<long long>(1024, (n + 255) / 256);

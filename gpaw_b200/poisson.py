@@ -586,9 +586,9 @@ def _mixed_result(self):
 
 
 def _mixed_prepare(self):
-    """Capture the solve now (synchronous; otherwise the first
-    solve_neutral_async does it)."""
-    check(self._h.lib.gb_mixed_prepare(self._h.h))
+    """Capture the solve now, for the solver's ``maxiter`` and ``correction``
+    (synchronous; otherwise the first solve_neutral_async does it)."""
+    check(self._h.lib.gb_mixed_prepare_for(self._h.h, int(self.maxiter)))
 
 
 MixedPoissonSolver.solve_neutral_async = _mixed_async

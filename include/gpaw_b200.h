@@ -410,9 +410,13 @@ GB_API int gb_mixed_result(gb_mixed* m, int* niter, double* rel_residual);
 /* Build the solver's captured solve now (what the first gb_mixed_solve_async
  * otherwise does): one uncaptured pass on the solver's own stream, then the
  * capture; synchronous.  Lets a host thread prepare solvers while another
- * thread enqueues solves of other solvers.  No counterpart in the
- * reference. */
+ * thread enqueues solves of other solvers.  gb_mixed_prepare builds all that
+ * a solve may need, gb_mixed_prepare_for what a solve of at most maxiter
+ * corrections needs (gb_mixed_set_correction), which gb_mixed_prepared tells
+ * to be there (1) or not (0).  No counterpart in the reference. */
 GB_API int gb_mixed_prepare(gb_mixed* m);
+GB_API int gb_mixed_prepare_for(gb_mixed* m, int maxiter);
+GB_API int gb_mixed_prepared(const gb_mixed* m, int maxiter);
 
 /* Many mixed-precision solves as one CUDA graph (no reference counterpart):
  * distinct solvers, grids of any sizes, each the solve of

@@ -86,6 +86,31 @@ def test_mixed_nonconvergence_raises(cuda):
     assert ps.niter == 2
 
 
+@pytest.mark.parametrize('kw', [
+    dict(), dict(maxiter=49), dict(correction='vcycle'),
+    dict(correction='direct', maxiter=3), dict(nn=4)])
+def test_prepare_builds_what_the_solve_runs(kw, cuda):
+    from gpaw_b200 import GridDescriptor, MixedPoissonSolver
+    gd = GridDescriptor((32, 40, 24), (5.0, 6.0, 4.0), 0)
+
+    def prepared(ps):
+        return ps._h.lib.gb_mixed_prepared(ps._h.h, ps.maxiter)
+
+    ps = MixedPoissonSolver(**kw)
+    ps.set_grid_descriptor(gd)
+    assert not prepared(ps)
+    ps.prepare()
+    assert prepared(ps)
+    phi, rho = gd.zeros(), gd.zeros()
+    rho[3, 4, 5], rho[20, 30, 10] = 1.0, -1.0
+    ps.solve_neutral(phi, rho)
+    # all limits at once, from C
+    ps = MixedPoissonSolver(**kw)
+    ps.set_grid_descriptor(gd)
+    assert ps._h.lib.gb_mixed_prepare(ps._h.h) == 0
+    assert all(ps._h.lib.gb_mixed_prepared(ps._h.h, n) for n in (1, 49, 50))
+
+
 def test_solver_pool_reuses_memory_and_results(cuda):
     """Solvers built through the library's caching allocator (gb_pool_*):
     a dropped solver's blocks are cached and handed to the next one of the

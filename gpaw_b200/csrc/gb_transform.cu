@@ -674,7 +674,9 @@ __device__ __forceinline__ T ip_value(const T* c, int stride, bool odd, const do
 // in a plane past a periodic edge of axis 0, multiply the in-grid cells by
 // that axis's phase.  `map` covers the whole batch; `b0` is this launch's
 // first grid in it.
-template <class T, int K, int TJ, int TK, int D, int LD>
+// SCALED: the values times oscale[grid] (a density's; as a run-time choice the
+// factor cost every other interpolation 2 to 7 %)
+template <class T, int K, int TJ, int TK, int D, int LD, bool SCALED>
 __global__ void __launch_bounds__(TJ * TK, 4)
 k_interpolate(const T* __restrict__ in, T* __restrict__ out, int nin, XferGeom G, Phases P,
               int chunk0, const __grid_constant__ CUtensorMap map, int b0,
@@ -911,13 +913,14 @@ k_interpolate(const T* __restrict__ in, T* __restrict__ out, int nin, XferGeom G
     // this thread's output column; fine plane f0 adds f0 * plane stride
     T* ocol = o + (long long)f1 * G.nout[2] + f2;
     const long long pstride = (long long)G.nout[1] * G.nout[2];
-    const double osc = oscale ? oscale[b] : 1.0;   // this grid's factor
+    double osc = 1.0;
+    if constexpr (SCALED) osc = oscale[b];
     auto emit = [&](int u, T v) {
         const int f0 = u - G.skip0[0];
         if (inside && f0 >= 0 && f0 < G.nout[0]) {
             T* dst = ocol + f0 * pstride;
             // accumulate: phi -= I(phi_coarse) (gpaw/poisson.py:520-521)
-            if (oscale) v = Num<T>::scale(v, osc);
+            if constexpr (SCALED) v = Num<T>::scale(v, osc);
             *dst = G.accumulate ? Num<T>::sub(*dst, v) : v;
         }
     };
@@ -1056,7 +1059,7 @@ static int launch_restrict_k(const void* in, void* out, void* out2, int nin, con
     return 0;
 }
 
-template <class T, int K, int LD>
+template <class T, int K, int LD, bool SCALED = false>
 static int launch_interp_v(const void* in, void* out, int nin, const XferGeom& G,
                            const Phases& P, cudaStream_t st, const double* oscale = nullptr) {
     constexpr int TK = sizeof(T) == 16 ? 16 : 32;
@@ -1075,7 +1078,7 @@ static int launch_interp_v(const void* in, void* out, int nin, const XferGeom& G
     }
     static bool attr = false;
     if (!attr) {
-        if (cudaFuncSetAttribute(k_interpolate<T, K, TJ, TK, D, LD>,
+        if (cudaFuncSetAttribute(k_interpolate<T, K, TJ, TK, D, LD, SCALED>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
             cudaSuccess)
             return -2;
@@ -1095,9 +1098,9 @@ static int launch_interp_v(const void* in, void* out, int nin, const XferGeom& G
         dim3 grid(t1 * t2, nchunks, nb);
         const long long ngin = (long long)G.g.n[0] * G.g.n[1] * G.g.n[2];
         const long long ngout = (long long)G.nout[0] * G.nout[1] * G.nout[2];
-        k_interpolate<T, K, TJ, TK, D, LD><<<grid, TJ * TK, smem, st>>>(
+        k_interpolate<T, K, TJ, TK, D, LD, SCALED><<<grid, TJ * TK, smem, st>>>(
             (const T*)in + b0 * ngin, (T*)out + b0 * ngout, nb, G, P, chunk0, map, b0,
-            oscale ? oscale + b0 : nullptr);
+            SCALED ? oscale + b0 : nullptr);
     }
     return 0;
 }
@@ -1191,10 +1194,10 @@ int launch_density(int k, const double* in, double* out, int nin, const XferGeom
     k_density_scale<<<nin, DENSITY_BLOCKS, 0, st>>>(work, k, dv, dvf, scale);
     const Phases P{};
     switch (k) {
-        case 2: return launch_interp_v<double, 2, 0>(in, out, nin, G, P, st, scale);
-        case 4: return launch_interp_v<double, 4, 0>(in, out, nin, G, P, st, scale);
-        case 6: return launch_interp_v<double, 6, 0>(in, out, nin, G, P, st, scale);
-        case 8: return launch_interp_v<double, 8, 0>(in, out, nin, G, P, st, scale);
+        case 2: return launch_interp_v<double, 2, 0, true>(in, out, nin, G, P, st, scale);
+        case 4: return launch_interp_v<double, 4, 0, true>(in, out, nin, G, P, st, scale);
+        case 6: return launch_interp_v<double, 6, 0, true>(in, out, nin, G, P, st, scale);
+        case 8: return launch_interp_v<double, 8, 0, true>(in, out, nin, G, P, st, scale);
     }
     return -1;
 }

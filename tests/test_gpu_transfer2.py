@@ -1,7 +1,6 @@
-"""Order-2 transfers of real grids against the oracle, bit for bit: the
-single-row form that small batches take and the four-row (two-row) form of
-large ones (from 1.2 million coarse points on), whose results on many copies
-of the same grids must equal the oracle's on each."""
+"""Order-2 transfers of real grids against the oracle, bit for bit, on small
+batches (short chunks) and on large ones (many CTAs, long chunks), whose
+results on many copies of the same grids must equal the oracle's on each."""
 import numpy as np
 import pytest
 

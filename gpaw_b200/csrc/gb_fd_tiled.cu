@@ -33,12 +33,13 @@
 namespace gb {
 
 
-// Planes per CTA along axis 0: the split with the least waves x planes, with
-// per_sm CTAs an SM at once (GPAW_B200_CTA_TARGET=n: n CTAs in all); a CTA
-// reads 2 nn planes beyond its own.  Against halving the chunk until the
-// launch had 296 CTAs: 32 x 111 x 119 x 95 real H psi 334 -> 294 us (two
-// chunks make 4.9 full waves instead of 2.4 of long ones).  The complex kernels
-// (per_sm 0) keep that older rule: 16 x 40 x 48 x 36, nn = 1, 14 us against 18.
+// Planes per CTA along axis 0, with per_sm CTAs an SM; a CTA reads 2 nn planes
+// beyond its own.  (GPAW_B200_CTA_TARGET=n: halved until the launch has n CTAs,
+// at least 2 nn planes.)
+// In us, halving until 296 CTAs, then the rule: complex 8 x 144^3 periodic
+// apply nn = 1 218, 164, nn = 3 312, 253; 16 x 96^3 residual nn = 1 228, 173;
+// real 8 x 143^3 kin psi + v psi nn = 3 285, 204; 24 x 111 x 119 x 99 apply nn =
+// 1 126, 112, nn = 3 206, 206.
 int cfd_chunk(const GridBC& g, int nn, int nin, int ty, int per_sm) {
     static int target = [] {
         const char* v = getenv("GPAW_B200_CTA_TARGET");
@@ -47,8 +48,8 @@ int cfd_chunk(const GridBC& g, int nn, int nin, int ty, int per_sm) {
     const int tiles_x = (g.n[2] + 31) / 32;
     const int tiles_y = (g.n[1] + ty - 1) / ty;
     const long long tiles = (long long)tiles_x * tiles_y * nin;
-    if (per_sm == 0) return halve_planes(g.n[0], 2 * nn, tiles, target > 0 ? target : 148 * 2);
-    return split_planes(g.n[0], 1, 2 * nn, tiles, target > 0 ? target : 148 * per_sm);
+    if (target > 0) return halve_planes(g.n[0], 2 * nn, tiles, target);
+    return balance_planes(g.n[0], 1, 2 * nn, tiles, per_sm, nn < 3 ? 0.2 : 0.12, 1.0);
 }
 
 // GPAW_B200_FMA=1 selects the fused-multiply-add form of the complex
@@ -623,6 +624,43 @@ static int cfd_wrapped_max(const GridBC& g, int NN, int TX, int TY) {
 
 bool tma_enabled();   // gb_transform.cu
 
+// Tile shapes (launch_cfd_nn says why): 32 columns a warp row.
+template <class T, int NN, int MODE>
+struct CfdShape {
+    static constexpr bool CPLX = sizeof(T) == 16, APPLY = MODE == EPI_APPLY;
+    static constexpr int TX = 32, TY = sizeof(T) == 4 ? 16 : 8;
+    static constexpr int RY = CPLX ? 1 : sizeof(T) == 8 ? 2 : (NN <= 3 && APPLY) ? 4 : 2;
+    static constexpr int D = CPLX ? 2 : NN == 3 ? 3 : 4;
+    static constexpr int ORD = (MODE == EPI_LIN && sizeof(T) == 8) ? 3 : 1;
+    static constexpr int MINB = CPLX ? ((NN <= 3 && (APPLY || MODE == EPI_POT)) ? 4 : 2)
+                                : sizeof(T) == 8 ? 4 : 512 / (32 * (16 / RY));
+};
+
+// CTAs an SM holds of that shape, in the form it mostly runs in (complex grids
+// by TMA); a launch in another form takes the same chunks, so that cfd_blocks
+// can count them
+template <class T, int NN, int MODE>
+static int cfd_per_sm() {
+    using S = CfdShape<T, NN, MODE>;
+    static const int n = [] {
+        constexpr int LD = S::CPLX ? 1 : 0, ST = NN + 1 + S::D;
+        const auto kernel =
+            k_fd_cfd<T, NN, S::TX, S::TY, S::RY, S::D, MODE, S::ORD, LD, S::MINB>;
+        constexpr int plane = (S::TX + 2 * NN) * (S::TY + 2 * NN);
+        constexpr int smem = ST * (LD ? (plane + 7) / 8 * 8 : plane) * (int)sizeof(T) +
+                             (LD ? ST * (int)sizeof(uint64_t) + 128 : 0);
+        int fit = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) !=
+                cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, kernel,
+                                                          S::TX * (S::TY / S::RY), smem) !=
+                cudaSuccess)
+            cudaGetLastError();
+        return fit > 0 ? fit : S::MINB;
+    }();
+    return n;
+}
+
 template <class T, int NN, int TX, int TY, int RY, int D, int MODE, int ORD, int LD, int MINB>
 static int launch_cfd_t(const void* in, void* out, int nin, const GridBC& g, const Phases& P,
                         const CfdStencil& cs, const Epi& ep, cudaStream_t st, int* nblk) {
@@ -649,7 +687,8 @@ static int launch_cfd_t(const void* in, void* out, int nin, const GridBC& g, con
     }
     const int tiles_x = (g.n[2] + TX - 1) / TX;
     const int tiles_y = (g.n[1] + TY - 1) / TY;
-    const int chunk0 = ep.chunk > 0 ? min(ep.chunk, g.n[0]) : cfd_chunk(g, NN, nin, TY, sizeof(T) == 16 ? 0 : 4);
+    const int chunk0 = ep.chunk > 0 ? min(ep.chunk, g.n[0])
+                                    : cfd_chunk(g, NN, nin, TY, cfd_per_sm<T, NN, MODE>());
     const int nch = (g.n[0] + chunk0 - 1) / chunk0;
     if (nblk) *nblk = tiles_x * tiles_y * nch;
     const long long ng = (long long)g.n[0] * g.n[1] * g.n[2];
@@ -666,7 +705,6 @@ static int launch_cfd_t(const void* in, void* out, int nin, const GridBC& g, con
     return 0;
 }
 
-// Tile shapes: 32 columns per warp row; f64 threads own 4 rows, complex 2.
 template <class T, int NN, int MODE>
 static int launch_cfd_nn(const void* in, void* out, int nin, const GridBC& g, const Phases& P,
                          const CfdStencil& cs, const Epi& ep, cudaStream_t st, int* nblk) {
@@ -675,14 +713,13 @@ static int launch_cfd_nn(const void* in, void* out, int nin, const GridBC& g, co
     if (!(cs.axis[0] == 2 && cs.axis[1] == 1 && cs.axis[2] == 0)) return -1;
     // rows per thread: fewer when the epilogue reads other arrays (their
     // prefetched values need registers too)
-    constexpr bool AUX = MODE != EPI_APPLY;
+    using S = CfdShape<T, NN, MODE>;
     if constexpr (sizeof(T) == 16) {
         // 32 x 8 tiles, one row a thread: 80 registers and 60 KB of ring
         // (nn = 3) let three CTAs share an SM; measured faster than 32 x 16
         // tiles of two rows a thread at two CTAs an SM (the rows' shared
         // axis-1 loads do not make up for the lost warps)
-        constexpr int D = NN <= 3 ? 2 : 2;
-        constexpr int MB = (NN <= 3 && (MODE == EPI_APPLY || MODE == EPI_POT)) ? 4 : 2;
+        constexpr int D = S::D, MB = S::MINB;
         if constexpr (MODE == EPI_APPLY && NN == 3)
             if (fused_apply())
                 return launch_cfd_t<T, NN, 32, 8, 1, D, MODE, 2, 0, MB>(in, out, nin, g, P, cs,
@@ -715,17 +752,16 @@ static int launch_cfd_nn(const void* in, void* out, int nin, const GridBC& g, co
         return launch_cfd_t<T, NN, 32, 8, 1, D, MODE, 1, 0, MB>(in, out, nin, g, P, cs, ep, st,
                                                                  nblk);
     } else {
-        constexpr int RY = (NN <= 3 && !AUX) ? 4 : 2;
         // nn = 3: three planes ahead makes the ring exactly 2nn+1 deep, so
         // every ring slot in the unrolled march is a constant
-        constexpr int D = NN == 3 ? 3 : 4;
+        constexpr int RY = S::RY, D = S::D;
         // float64: 32 x 8 tiles of two rows a thread (128 threads, more
         // CTAs an SM) measured faster than 32 x 16 tiles (nn = 3 apply
         // 14 %, preconditioner 9 %, FP64 V-cycles 3-7 %)
         // split sums for the FP64 defect of the mixed solver (measured
         // faster there); the FP32 levels keep one chain (measured slower
         // with three: more registers)
-        constexpr int ORDL = (MODE == EPI_LIN && sizeof(T) == 8) ? 3 : 1;
+        constexpr int ORDL = S::ORD;
         if constexpr (MODE == EPI_LIN) {
             // tile shapes of the mixed solver's passes under measurement
             // (GPAW_B200_LIN_VARIANT): 1 = one row a thread, 32 x 8 tiles
@@ -750,10 +786,7 @@ static int launch_cfd_nn(const void* in, void* out, int nin, const GridBC& g, co
                         in, out, nin, g, P, cs, ep, st, nblk);
             }
         }
-        if constexpr (sizeof(T) == 8)
-            return launch_cfd_t<T, NN, 32, 8, 2, D, MODE, ORDL, 0, 4>(in, out, nin, g, P, cs, ep,
-                                                                      st, nblk);
-        return launch_cfd_t<T, NN, 32, 16, RY, D, MODE, ORDL, 0, 512 / (32 * (16 / RY))>(
+        return launch_cfd_t<T, NN, S::TX, S::TY, RY, D, MODE, ORDL, 0, S::MINB>(
             in, out, nin, g, P, cs, ep, st, nblk);
     }
 }
@@ -805,13 +838,26 @@ template int launch_fd_cfd<double2>(int, const void*, void*, int, const GridBC&,
 template int launch_fd_cfd<float>(int, const void*, void*, int, const GridBC&, const Phases&,
                                   const CfdStencil&, int, const Epi&, cudaStream_t, int*);
 
-// Number of CTAs per grid of the EPI_RESID launch (partials per grid).
-int cfd_blocks(const GridBC& g, int nn, int elem_bytes, int nin, int chunk) {
-    // the tile of launch_cfd_nn: 32 x 16 for float, 32 x 8 otherwise
-    const int TX = 32, TY = elem_bytes == 4 ? 16 : 8;
-    const int tiles_x = (g.n[2] + TX - 1) / TX;
-    const int tiles_y = (g.n[1] + TY - 1) / TY;
-    const int chunk0 = chunk > 0 ? std::min(chunk, g.n[0]) : cfd_chunk(g, nn, nin, TY, elem_bytes == 16 ? 0 : 4);
+template <class T, int MODE>
+static int cfd_per_sm_nn(int nn) {
+    switch (nn) {
+        case 1: return cfd_per_sm<T, 1, MODE>();
+        case 2: return cfd_per_sm<T, 2, MODE>();
+        case 3: return cfd_per_sm<T, 3, MODE>();
+        case 4: return cfd_per_sm<T, 4, MODE>();
+        case 5: return cfd_per_sm<T, 5, MODE>();
+    }
+    return cfd_per_sm<T, 6, MODE>();
+}
+
+// Number of CTAs a grid of a launch that writes partial sums: EPI_RESID of a
+// double or complex grid, or EPI_LIN of a double one (their 32 x 8 tiles).
+int cfd_blocks(int mode, const GridBC& g, int nn, int elem_bytes, int nin, int chunk) {
+    const int tiles_x = (g.n[2] + 31) / 32, tiles_y = (g.n[1] + 7) / 8;
+    const int per_sm = mode == EPI_LIN     ? cfd_per_sm_nn<double, EPI_LIN>(nn)
+                       : elem_bytes == 16 ? cfd_per_sm_nn<double2, EPI_RESID>(nn)
+                                          : cfd_per_sm_nn<double, EPI_RESID>(nn);
+    const int chunk0 = chunk > 0 ? std::min(chunk, g.n[0]) : cfd_chunk(g, nn, nin, 8, per_sm);
     return tiles_x * tiles_y * ((g.n[0] + chunk0 - 1) / chunk0);
 }
 

@@ -14,8 +14,9 @@
 // point: 25 taps of a hexagonal cell's nn = 3 Laplacian take 3.1 clocks of an
 // SM a point, against 1.4 for its HBM traffic), so the other work of a tap
 // has to be small.  A CTA owns a column tile of up to 512 points (its sides
-// divide the plane evenly) and a chunk of planes along axis 0; planes with their halo (corners too) stream by cp.async into
-// a ring of 2 R + 2 stages.  A thread owns two points of the tile, so a
+// divide the plane evenly) and a chunk of planes along axis 0; planes with
+// their halo (corners too) stream by cp.async into a ring of 2 R + 2 stages.
+// A thread owns two points of the tile, so a
 // tap's address (its byte offset from a kernel parameter, wrapped at the
 // ring's end by one unsigned minimum) serves both.  Wrap-around is folded
 // into the copy's source, and Bloch phases are applied once a cell, right
@@ -242,7 +243,8 @@ struct Geom {
 // (two a thread) whose staged plane fits, with the least work: a tap reads
 // shared memory for all 512 points, a staged cell is written once.  (A fixed
 // 32 x 16 tile computes 1.42 times the points of a 72 x 100 plane.)  Chunk of
-// axis 0: least waves x planes.
+// axis 0: least waves x planes (24 x 72 x 72 x 100 hexagonal 274 us; 294 with the
+// stencils' share and half a wave for an unfinished one).
 Geom geom(const GridBC& g, int R, int ncoefs, int nin, int cells, int blocks) {
     Geom G{};
     long long best = -1;
@@ -264,7 +266,7 @@ Geom geom(const GridBC& g, int R, int ncoefs, int nin, int cells, int blocks) {
     }
     G.tiles_x = (g.n[2] + G.tw - 1) / G.tw;
     G.tiles = G.tiles_x * ((g.n[1] + G.th - 1) / G.th);
-    G.chunk = split_planes(g.n[0], 1, 2 * R, (long long)G.tiles * nin, 148 * blocks);
+    G.chunk = balance_planes(g.n[0], 1, 2 * R, (long long)G.tiles * nin, blocks, 0.0, 1.0);
     G.nchunk = (g.n[0] + G.chunk - 1) / G.chunk;
     return G;
 }

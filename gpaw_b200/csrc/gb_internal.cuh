@@ -109,14 +109,14 @@ template <class T>
 int launch_fd_cfd(int mode, const void* in, void* out, int nin, const GridBC& g,
                   const Phases& P, const CfdStencil& cs, int nn, const Epi& ep,
                   cudaStream_t st, int* nblk);
-int cfd_blocks(const GridBC& g, int nn, int elem_bytes, int nin, int chunk = 0);
+int cfd_blocks(int mode, const GridBC& g, int nn, int elem_bytes, int nin, int chunk = 0);
 // the passes for general stencils up to range 6 (gb_general.cu): 0, -1 not
 // taken, -2 the shared-memory limit could not be raised
 template <class T>
 int launch_general(int mode, const void* in, void* out, int nin, const GridBC& g,
                    const Phases& P, const Stencil& st, const Epi& ep, cudaStream_t stream);
 int general_blocks(const GridBC& g, int range, int ncoefs, int nin, int elem_bytes);
-int cfd_chunk(const GridBC& g, int nn, int nin, int ty, int per_sm = 4);
+int cfd_chunk(const GridBC& g, int nn, int nin, int ty, int per_sm);
 // read and clear the device fault flag of a kernel file (bounded waits)
 int take_fault_transform(int* code);
 int take_fault_cfd(int* code);

@@ -1395,7 +1395,7 @@ extern "C" int gb_mixed_new(int nlevels, gb_operator* op64, gb_operator* const* 
     // takes the level-0 operator, else of the plane-marching kernel
     m->nres = (pass_on() && pass_supported_grid(op64->g, op64->cs, op64->nn))
                   ? pass_blocks(op64->g, 8)
-                  : op_resid_blocks(op64, 1, 8);
+                  : op_resid_blocks(op64, 1, 8, EPI_LIN);
     m->nblk64 = std::max(m->nres, 1024);
     if (ce == cudaSuccess) ce = pool_malloc(&m->x, nc);
     if (ce == cudaSuccess) ce = pool_malloc(&m->r, nc);

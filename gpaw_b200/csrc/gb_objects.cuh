@@ -132,10 +132,11 @@ namespace gb {
 
 // ----------------------------------------------------------------- Operator
 
-// Partial sums produced per grid by a residual sweep of `op`.
-inline int op_resid_blocks(const gb_operator* op, int nin, int es) {
-    return op->tiled ? cfd_blocks(op->g, op->nn, es, nin, op->chunk) 
-           : op->general ? general_blocks(op->g, op->st.range, op->st.ncoefs, nin, es) : residual_blocks(op->g);
+// Partial sums produced per grid by a sweep of `op` in a mode that writes them.
+inline int op_resid_blocks(const gb_operator* op, int nin, int es, int mode = EPI_RESID) {
+    if (op->tiled) return cfd_blocks(mode, op->g, op->nn, es, nin, op->chunk);
+    if (op->general) return general_blocks(op->g, op->st.range, op->st.ncoefs, nin, es);
+    return residual_blocks(op->g);
 }
 
 // One pass of the stencil with a fused epilogue; plane-marching kernel for

@@ -8,9 +8,9 @@
 // and marches along axis 0; a lane reads its own columns of the three fine
 // rows (restriction) or its two coarse columns of two rows (interpolation)
 // straight into registers, all of a plane at once, so that many loads are in
-// flight, and keeps the in-plane results of the last plane.  One row a lane at every size: four for the
-// restriction and two for the interpolation of large batches read less twice,
-// but leave fewer warps to hide the loads.
+// flight, and keeps the in-plane results of the last plane.  One row a lane at
+// every size: four for the restriction and two for the interpolation of large
+// batches read less twice, but leave fewer warps to hide the loads.
 // Restriction / interpolation in us, general kernels, then several rows, now:
 // 128 x 111^3 366 / 466, 347 / 336, 316 / 305; 16 x 96^3 periodic 45 / 41,
 // 55 / 39, 39 / 35; 64 x 48 x 64 x 80 periodic 52 / 53, 55 / 41, 50 / 38.
@@ -200,7 +200,7 @@ void run_restrict(const double* in, double* out, double* out2, int nin, const Xf
     const int tiles = tiles2 * ((G.nout[1] + 7) / 8);
     const int chunk = G.chunk > 0
                           ? std::min(G.chunk, G.nout[0])
-                          : balance_planes(G.nout[0], 2, 1, (long long)tiles * nin, 4, 0.25);
+                          : balance_planes(G.nout[0], 2, 1, (long long)tiles * nin, 4, 0.25, 0.5);
     const long long ngin = (long long)G.g.n[0] * G.g.n[1] * G.g.n[2];
     const long long ngout = (long long)G.nout[0] * G.nout[1] * G.nout[2];
     for (int b0 = 0; b0 < nin; b0 += 65535)
@@ -215,7 +215,8 @@ void run_interp(const double* in, double* out, int nin, const XferGeom& G, cudaS
     const int tiles2 = (pairs[2] + 31) / 32;
     const int tiles = tiles2 * ((pairs[1] + 7) / 8);
     const int chunk = G.chunk > 0 ? std::min(G.chunk, pairs[0])
-                                  : balance_planes(pairs[0], 1, 1, (long long)tiles * nin, 3, 0.4);
+                                  : balance_planes(pairs[0], 1, 1, (long long)tiles * nin, 3,
+                                                   0.4, 0.5);
     const long long ngin = (long long)G.g.n[0] * G.g.n[1] * G.g.n[2];
     const long long ngout = (long long)G.nout[0] * G.nout[1] * G.nout[2];
     for (int b0 = 0; b0 < nin; b0 += 65535)

@@ -619,11 +619,18 @@ static int launch_restrict_tma_v(const void* in, void* out, void* out2, int nin,
         attr = true;
     }
     const int t1 = (G.nout[1] + TJ - 1) / TJ, t2 = (G.nout[2] + TK - 1) / TK;
-    // two fine planes an output plane, 2 K - 3 more to start with (and the
-    // set-up of a CTA, some eight planes' time)
-    const int chunk0 = G.chunk > 0 ? std::min(G.chunk, G.nout[0])
-                                   : split_planes(G.nout[0], 2, 2 * K - 3 + 8,
-                                                  (long long)t1 * t2 * nin, 148 * MINB);
+    // two fine planes an output plane, 2 K - 3 more to start with, and the
+    // set-up of a CTA: two planes' time, eight of the short ones of K = 2,
+    // whose CTAs do not slow each other (16 x 40 x 48 x 36 periodic: 21 us so,
+    // 25 by the others' constants; 16 x 80 x 96 x 72 67 and 69)
+    // In us, halving until 592 CTAs, then least waves x planes, then this rule:
+    // 4 x 47 x 63 x 55, order 8, 29, 47, 29; 8 x 143^3, order 6, 175, 197, 175
+    constexpr bool SHORT = K == 2;
+    const int chunk0 = G.chunk > 0
+                           ? std::min(G.chunk, G.nout[0])
+                           : balance_planes(G.nout[0], 2, 2 * K - 3 + (SHORT ? 8 : 2),
+                                            (long long)t1 * t2 * nin, MINB, SHORT ? 0.0 : 0.25,
+                                            SHORT ? 1.0 : 0.5);
     const int nchunks = (G.nout[0] + chunk0 - 1) / chunk0;
     for (int b0 = 0; b0 < nin; b0 += 65535) {
         const int nb = min(65535, nin - b0);
@@ -1037,15 +1044,16 @@ static int launch_restrict_k(const void* in, void* out, void* out2, int nin, con
         attr = true;
     }
     const int t1 = (G.nout[1] + TJ - 1) / TJ, t2 = (G.nout[2] + TK - 1) / TK;
-    // (three CTAs an SM, fewer where their shared memory is large; complex
-    // grids keep many short chunks: 16 x 80 x 96 x 72, K = 2, 43 us against
-    // 46)
+    // (three CTAs an SM, fewer where their shared memory is large)
     const int per_sm = std::max(1, std::min(3, (int)(227 * 1024 / (smem + 1024))));
     const long long tiles = (long long)t1 * t2 * nin;
-    const int chunk0 = G.chunk > 0 ? std::min(G.chunk, G.nout[0])
-                       : sizeof(T) == 16 ? halve_planes(G.nout[0], 4, tiles, 148 * 4)
-                                         : split_planes(G.nout[0], 2, 2 * K - 3 + 8, tiles,
-                                                        148 * per_sm);
+    // (K = 2 of complex grids, whose ragged tiles end early: many short chunks,
+    // 16 x 40 x 48 x 36 periodic 21 us, by the others' rule 25)
+    const int chunk0 =
+        G.chunk > 0 ? std::min(G.chunk, G.nout[0])
+        : sizeof(T) == 16 && K == 2
+            ? halve_planes(G.nout[0], 4, tiles, 148 * 4)
+            : balance_planes(G.nout[0], 2, 2 * K - 1, tiles, per_sm, 0.25, 0.5);
     const int nchunks = (G.nout[0] + chunk0 - 1) / chunk0;
     for (int b0 = 0; b0 < nin; b0 += 65535) {
         const int nb = min(65535, nin - b0);
@@ -1087,11 +1095,9 @@ static int launch_interp_v(const void* in, void* out, int nin, const XferGeom& G
     const int t1 = (G.nout[1] + TJ - 1) / TJ, t2 = (G.nout[2] + TK - 1) / TK;
     const int n0p = G.s[0] - (K - 1) + G.skip1[0];
     const int per_sm = std::max(1, std::min(4, (int)(227 * 1024 / (smem + 1024))));
-    // (complex: as for the restriction, 28 us against 30)
     const long long tiles = (long long)t1 * t2 * nin;
     const int chunk0 = G.chunk > 0 ? std::min(G.chunk, n0p)
-                       : sizeof(T) == 16 ? halve_planes(n0p, 4, tiles, 148 * 8)
-                                         : split_planes(n0p, 1, K - 1 + 8, tiles, 148 * per_sm);
+                                   : balance_planes(n0p, 1, K - 1, tiles, per_sm, 0.25, 0.5);
     const int nchunks = (n0p + chunk0 - 1) / chunk0;
     for (int b0 = 0; b0 < nin; b0 += 65535) {
         const int nb = min(65535, nin - b0);

@@ -509,7 +509,16 @@ static int launch_wfd_tiled_k(const void* in, void* out, int nin, const GridBC& 
     }
     const int tiles_x = (g.n[2] + WX - 1) / WX;
     const int tiles_y = (g.n[1] + WY - 1) / WY;
-    const int chunk0 = cfd_chunk(g, R, nin, WY, sizeof(T) == 16 ? 0 : 4);
+    static const int per_sm = [] {
+        int fit = 0;
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                &fit, k_wfd_tiled<T, R, S, GR, MODE>, WX * WY, smem) != cudaSuccess)
+            cudaGetLastError();
+        // (a fifth CTA shares the weights' lines less well: 8 x 143^3 real 386
+        // us with chunks for four, 411 for five)
+        return fit > 0 ? std::min(fit, 4) : 2;
+    }();
+    const int chunk0 = cfd_chunk(g, R, nin, WY, per_sm);
     const int nch = (g.n[0] + chunk0 - 1) / chunk0;
     const long long ng = (long long)g.n[0] * g.n[1] * g.n[2];
     for (int b0 = 0; b0 < nin; b0 += 65535) {

@@ -52,6 +52,7 @@ SIGNATURES = {
     'gb_mixed_prepare_for': (C.c_int, [_p, C.c_int]),
     'gb_mixed_prepared': (C.c_int, [_p, C.c_int]),
     'gb_mixed_set_correction': (C.c_int, [_p, C.c_int]),
+    'gb_mixed_direct_eager': (C.c_int, [_p, _p, _p, _p]),
     'gb_mixed_vcycle_eager': (C.c_int, [_p, _p, _p, _p]),
     'gb_mixed_set_fused_coarse': (C.c_int, [_p, C.c_int]),
     'gb_trace_end': (C.c_int, [C.c_int, C.POINTER(C.c_float),

@@ -619,6 +619,13 @@ int DirectGroup::solve(double* phi, const double* rho, double tol, int maxiter,
     return run(st);
 }
 
+int DirectGroup::eager(double* phi, const double* rho, cudaStream_t st) {
+    k_direct_set<<<1, 1, 0, st>>>(grids, ctl, phi, rho, 0.0, 1);
+    if (int rc = group_defect(*this, 0, nullptr, st)) return rc;
+    if (int rc = group_correction(*this, st)) return rc;
+    return group_defect(*this, 1, nullptr, st);
+}
+
 int DirectGroup::solve_batch(double* const* user, double tol, int maxiter, cudaStream_t st) {
     k_direct_set_batch<<<(n + 127) / 128, 128, 0, st>>>(grids, ctl, user, n, tol, maxiter);
     GB_LAUNCH_CHECK();

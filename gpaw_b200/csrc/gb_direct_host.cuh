@@ -38,6 +38,7 @@ struct DirectGroup {
     int capture(cudaStream_t cs);
     int run(cudaStream_t st);
     int solve(double* phi, const double* rho, double tol, int maxiter, cudaStream_t st);
+    int eager(double* phi, const double* rho, cudaStream_t st);
     int solve_batch(double* const* user, double tol, int maxiter, cudaStream_t st);
 };
 

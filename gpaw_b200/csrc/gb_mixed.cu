@@ -1673,6 +1673,17 @@ extern "C" int gb_mixed_vcycle_eager(gb_mixed* m, double* phi, const double* rho
     return 0;
 }
 
+extern "C" int gb_mixed_direct_eager(gb_mixed* m, double* phi, const double* rho,
+                                     void* stream) {
+    if (!m || !phi || !rho) return fail(GB_EINVAL, "mixed direct: NULL argument");
+    if (!m->dtab) return fail(GB_EINVAL, "mixed direct: this solver has no direct correction");
+    if (ranges_overlap(phi, rho, (size_t)m->op64->ng() * sizeof(double)))
+        return fail(GB_EINVAL, "mixed direct: phi and rho overlap");
+    if (!m->dgrp)
+        if (int rc = build_direct_group(m)) return rc;
+    return m->dgrp->eager(phi, rho, (cudaStream_t)stream);
+}
+
 extern "C" int gb_mixed_solve(gb_mixed* m, double* phi, const double* rho, double tol,
                               int maxiter, int* niter, double* rel_residual, void* stream) {
     if (int rc = gb_mixed_solve_async(m, phi, rho, tol, maxiter, stream)) return rc;

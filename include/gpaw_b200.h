@@ -386,6 +386,8 @@ GB_API int gb_mixed_set_correction(gb_mixed* m, int correction);
  * phi <- phi + V32(rho - L phi).  For profilers and kernel traces (its
  * kernels carry gb_trace labels); no counterpart in the reference. */
 GB_API int gb_mixed_vcycle_eager(gb_mixed* m, double* phi, const double* rho, void* stream);
+/* The same for one direct correction (phi and rho apart). */
+GB_API int gb_mixed_direct_eager(gb_mixed* m, double* phi, const double* rho, void* stream);
 
 /* Solve until ||rho - L phi|| / ||rho|| <= tol (both norms in FP64, on the
  * device), starting from phi; at most maxiter V-cycles (GB_ENOCONV

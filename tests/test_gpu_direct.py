@@ -72,6 +72,21 @@ def test_direct_against_dense_solution(pbc, cuda):
     assert np.linalg.norm(to_np(phi) - ref) <= 1e-10 * np.linalg.norm(ref)
 
 
+def test_eager_correction_equals_the_solve(cuda):
+    """The form for profilers, kernel by kernel."""
+    import ctypes as C
+    import torch
+    gd, ps, gdo = _solver((24, 32, 100), 0)
+    rho = to_dev(np.random.default_rng(7).standard_normal(tuple(gdo.n_c)))
+    phi, got = gd.zeros(), gd.zeros()
+    assert ps.solve_neutral(phi, rho) == 1
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    assert ps._h.lib.gb_mixed_direct_eager(
+        ps._h.h, C.c_void_p(got.data_ptr()), C.c_void_p(rho.data_ptr()),
+        st) == 0
+    assert torch.equal(got, phi)
+
+
 def test_the_caller_chooses_the_correction(cuda):
     """Direct under a low limit, V-cycles under a high one; a grid without a
     direct correction is refused."""

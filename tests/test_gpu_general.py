@@ -1,6 +1,6 @@
 """The tiled kernel for general stencils against the oracle, bit for bit (the
-same operations in the same order), at the edges of its 32 x 16 tiles, every
-range it takes and one it does not."""
+same operations in the same order), at planes that its tiles divide evenly
+or not, every range it takes and one it does not."""
 import numpy as np
 import pytest
 

@@ -206,7 +206,8 @@ __device__ __forceinline__ void restrict_to(const CoarseLevel& F, const CoarseLe
 #pragma unroll
                 for (int e = 0; e < 3; e++)
                     v[a][b][e] = (j[0][a] | j[1][b] | j[2][e]) < 0
-                                     ? 0.0 : get<LOCAL>(A + (j[0][a] * n1 + j[1][b]) * n2 + j[2][e]);
+                                     ? 0.0
+                                     : get<LOCAL>(A + (j[0][a] * n1 + j[1][b]) * n2 + j[2][e]);
         double u[3];
 #pragma unroll
         for (int a = 0; a < 3; a++) {
